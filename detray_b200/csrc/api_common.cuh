@@ -6,7 +6,9 @@
 
 #include <cuda_runtime.h>
 
+#include <mutex>
 #include <string>
+#include <vector>
 
 #include "core/propagate.cuh"
 #include "detray_b200/dprop.h"
@@ -20,6 +22,49 @@ dprop_status cuda_fail(cudaError_t e, const char* what);
 // Register budget of a launch: resident CTAs of 128 threads per SM, one of
 // 8 (64 registers), 12 (40) or 16 (32).
 int occupancy_of(const dprop_launch* lc);
+
+// Device memory the library keeps between calls: one grow-only buffer per
+// device, shared by all callers.  A call holds it (use) from take() until its
+// work is enqueued, so that calls of several host threads do not interleave,
+// and its work starts after that of the call before it, on whichever stream
+// that was: calls on several streams that need the same buffer run one after
+// the other, they do not overwrite each other.
+class kept_scratch {
+    struct slot {
+        void* buf{nullptr};
+        size_t bytes{0};
+        cudaEvent_t last{nullptr};  // the last call's work on the buffer
+        bool captured{false};       // a stream capture holds its address
+    };
+
+public:
+    class use {
+    public:
+        use() = default;
+        use(const use&) = delete;
+        use& operator=(const use&) = delete;
+        ~use();
+        void* buf{nullptr};
+
+    private:
+        friend class kept_scratch;
+        std::unique_lock<std::mutex> lock_;
+        cudaEvent_t last_{nullptr};  // recorded at the end (not in a capture)
+        cudaStream_t stream_{nullptr};
+    };
+
+    // At least `bytes` on the current device for work on `stream`.  Inside a
+    // stream capture the captured work is not ordered against other calls
+    // (an event from outside a capture cannot be waited for in it).
+    cudaError_t take(size_t bytes, cudaStream_t stream, use* u);
+    // Frees the buffers of all devices.
+    void release();
+
+private:
+    std::mutex mutex_;
+    std::vector<slot> slots_;      // by device
+    std::vector<void*> retired_;   // outgrown, but in a captured graph
+};
 
 // Number of a new detector or field handle, never given twice: a cached
 // CUDA graph is matched by it, since the address of a destroyed handle may be

@@ -47,6 +47,85 @@ uint64_t next_handle_id() {
     return ++last;
 }
 
+kept_scratch::use::~use() {
+    if (last_) {
+        cudaEventRecord(last_, stream_);
+    }
+}
+
+cudaError_t kept_scratch::take(size_t bytes, cudaStream_t stream, use* u) {
+    std::unique_lock<std::mutex> lock(mutex_);
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) {
+        return e;
+    }
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if ((e = cudaStreamIsCapturing(stream, &cap)) != cudaSuccess) {
+        return e;
+    }
+    const bool capturing = cap != cudaStreamCaptureStatusNone;
+    if (slots_.size() <= static_cast<size_t>(dev)) {
+        slots_.resize(static_cast<size_t>(dev) + 1u);
+    }
+    slot& s = slots_[static_cast<size_t>(dev)];
+    if (s.bytes < bytes) {
+        if (s.buf && capturing) {
+            return cudaErrorStreamCaptureUnsupported;
+        }
+        if (s.buf && s.captured) {
+            retired_.push_back(s.buf);
+        } else if (s.buf) {
+            if (s.last && (e = cudaEventSynchronize(s.last)) != cudaSuccess) {
+                return e;
+            }
+            cudaFree(s.buf);
+        }
+        s.buf = nullptr;
+        s.bytes = 0;
+        s.captured = false;
+        if ((e = cudaMalloc(&s.buf, bytes)) != cudaSuccess) {
+            s.buf = nullptr;
+            cudaGetLastError();
+            return e;
+        }
+        s.bytes = bytes;
+    }
+    if (capturing) {
+        s.captured = true;
+    } else {
+        if (!s.last) {
+            e = cudaEventCreateWithFlags(&s.last, cudaEventDisableTiming);
+        } else {
+            e = cudaStreamWaitEvent(stream, s.last, 0);
+        }
+        if (e != cudaSuccess) {
+            return e;
+        }
+        u->last_ = s.last;
+        u->stream_ = stream;
+    }
+    u->buf = s.buf;
+    u->lock_ = std::move(lock);
+    return cudaSuccess;
+}
+
+void kept_scratch::release() {
+    std::lock_guard<std::mutex> lock(mutex_);
+    for (slot& s : slots_) {
+        if (s.last) {
+            cudaEventSynchronize(s.last);
+            cudaEventDestroy(s.last);
+        }
+        cudaFree(s.buf);
+        s = slot{};
+    }
+    for (void* p : retired_) {
+        cudaFree(p);
+    }
+    retired_.clear();
+}
+
 dprop_status cuda_fail(cudaError_t e, const char* what) {
     g_last_error = std::string(what) + ": " + cudaGetErrorString(e);
     return (e == cudaErrorMemoryAllocation) ? DPROP_E_OOM : DPROP_E_CUDA;
@@ -98,14 +177,12 @@ dprop_status ensure_scratch(size_t bytes) {
     return DPROP_OK;
 }
 
-// Library-owned device scratch of the direction sort and of the persistent
-// method (grow-only).
-struct sort_scratch {
-    void* buf{nullptr};
-    size_t bytes{0};
-};
-sort_scratch g_sort;
-sort_scratch g_rounds;
+// Kept between calls: the direction sort's scratch, the slots and queues of the
+// persistent method, the staged results of sorted plain propagations.  A call
+// that needs two of them takes them in this order.
+dprop::api::kept_scratch g_sort;
+dprop::api::kept_scratch g_rounds;
+dprop::api::kept_scratch g_stage;
 
 // Sort key of a track, 20 bits: 7 bits of theta (major), 8 bits of phi, the
 // charge sign and 4 bits of log10(pT / GeV) over [-1, 2].  Tracks that share
@@ -622,44 +699,24 @@ dprop_status launch(const dprop_config& c, const dprop_launch* launch_cfg,
     };
     if (!(launch_cfg && launch_cfg->use_graph)) {
         launch_scratch scr{};
+        dprop::api::kept_scratch::use sort_use, work_use;
         if (plan.sort) {
-            const size_t need = sort_scratch_bytes(n);
-            if (g_sort.bytes < need) {
-                if (g_sort.buf) {
-                    DPROP_CUDA(cudaStreamSynchronize(stream));
-                    cudaFree(g_sort.buf);
-                    g_sort.buf = nullptr;
-                    g_sort.bytes = 0;
-                }
-                DPROP_CUDA(cudaMalloc(&g_sort.buf, need));
-                g_sort.bytes = need;
-            }
-            scr.sort = g_sort.buf;
-            scr.sort_bytes = need;
+            scr.sort_bytes = sort_scratch_bytes(n);
+            DPROP_CUDA(g_sort.take(scr.sort_bytes, stream, &sort_use));
+            scr.sort = sort_use.buf;
         }
-        const size_t need = work_bytes();
-        if (need > 0) {
-            if (g_rounds.bytes < need) {
-                if (g_rounds.buf) {
-                    DPROP_CUDA(cudaStreamSynchronize(stream));
-                    cudaFree(g_rounds.buf);
-                    g_rounds.buf = nullptr;
-                    g_rounds.bytes = 0;
-                }
-                const cudaError_t e = cudaMalloc(&g_rounds.buf, need);
-                if (e == cudaErrorMemoryAllocation && !plan.rounds) {
-                    // staging is an option: without room for it the results
-                    // go to the caller's arrays directly
-                    cudaGetLastError();
-                    g_rounds.buf = nullptr;
-                    plan.stage_cap = 0u;
-                } else {
-                    DPROP_CUDA(e);
-                    g_rounds.bytes = need;
-                }
+        scr.rounds_bytes = work_bytes();
+        if (scr.rounds_bytes > 0) {
+            const cudaError_t e = (plan.rounds ? g_rounds : g_stage)
+                                      .take(scr.rounds_bytes, stream, &work_use);
+            if (e == cudaErrorMemoryAllocation && !plan.rounds) {
+                // staging is an option: without room for it the results go
+                // to the caller's arrays directly
+                plan.stage_cap = 0u;
+            } else {
+                DPROP_CUDA(e);
             }
-            scr.rounds = g_rounds.buf;
-            scr.rounds_bytes = g_rounds.bytes;
+            scr.rounds = work_use.buf;
         }
         return enqueue_propagation<In>(c, launch_cfg, plan, det, field, io, n,
                                        stream, scr);
@@ -1765,10 +1822,9 @@ dprop_status dprop_release_cache(void) {
         destroy_entry(e);
     }
     g_graphs.clear();
-    cudaFree(g_sort.buf);
-    g_sort = sort_scratch{};
-    cudaFree(g_rounds.buf);
-    g_rounds = sort_scratch{};
+    g_sort.release();
+    g_rounds.release();
+    g_stage.release();
     cudaFree(g_scratch.buf);
     g_scratch.buf = nullptr;
     g_scratch.bytes = 0;

@@ -407,7 +407,14 @@ dprop_status dprop_field_destroy(dprop_field* field);
 
 /* Propagate n tracks whose parameters and results live in device memory.
  * Stream ordered; returns once the work is enqueued on `stream`
- * (a cudaStream_t, or NULL for the legacy default stream). */
+ * (a cudaStream_t, or NULL for the legacy default stream).
+ *
+ * Sorted calls and the persistent method work in scratch the library keeps
+ * per device.  Calls on different streams, or from different host threads,
+ * that need the same scratch are ordered one after the other on the device.
+ * Work captured into a caller's own CUDA graph is not: the caller orders the
+ * replays of such a graph against other sorted or persistent calls.  (Graphs
+ * of use_graph own their scratch.) */
 dprop_status dprop_propagate(const dprop_config* cfg,
                              const dprop_launch* launch,
                              const dprop_detector* det,

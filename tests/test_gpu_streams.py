@@ -1,0 +1,82 @@
+"""Calls on several streams, and from several host threads, that share the
+library's kept scratch (direction sort, persistent method, staged results):
+each gets the results of a call made alone, bit for bit."""
+import threading
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+N = 40000
+FORMS = {
+    "rounds": dict(method=1, ctas_per_sm=3),
+    "rounds_sorted": dict(method=1, ctas_per_sm=3, sort_tracks=1),
+    "plain_sorted": dict(sort_tracks=1),
+}
+
+
+@pytest.fixture(scope="module")
+def setup():
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from detray_b200 import abi, geometry, propagator, tracks
+    from detray_b200.units import T
+    det = propagator.Detector(geometry.load_geometry("toy_4brl_7edc"))
+    field = propagator.Field.constant((0.0, 0.0, 2.0 * T))
+    cfg = abi.make_config(max_records=24, search_window=(3, 3),
+                          estimate_scattering_noise=0)
+    trk = [torch.tensor(tracks.toy_tracks(N, seed=s), dtype=torch.float32,
+                        device="cuda") for s in (31, 32)]
+
+    def call(side, form, res, stream=None):
+        propagator.propagate(cfg, det, field, trk[side], results=res,
+                             launch=propagator.make_launch(**FORMS[form]),
+                             stream=stream)
+
+    def results():
+        r = propagator.alloc_device_results(N, cfg.max_records, "cuda")
+        for t in r.tensors.values():
+            t.zero_()
+        return r
+
+    return torch, call, results
+
+
+@pytest.mark.parametrize("threads", [False, True],
+                         ids=["streams", "threads"])
+@pytest.mark.parametrize("forms", [
+    ("rounds", "plain_sorted"), ("plain_sorted", "plain_sorted"),
+    ("rounds_sorted", "rounds_sorted"), ("rounds", "rounds")])
+def test_overlapping_calls(setup, forms, threads):
+    torch, call, results = setup
+    alone, got, streams = [], [], []
+    for side, form in enumerate(forms):
+        r = results()
+        call(side, form, r)
+        torch.cuda.synchronize()
+        alone.append(r)
+        got.append([results() for _ in range(4)])
+        streams.append(torch.cuda.Stream())
+    torch.cuda.synchronize()
+
+    def run(side):
+        for r in got[side]:
+            call(side, forms[side], r, streams[side])
+
+    if threads:
+        ts = [threading.Thread(target=run, args=(s,)) for s in (0, 1)]
+        for t in ts:
+            t.start()
+        for t in ts:
+            t.join()
+    else:
+        for k in range(4):
+            for side in (0, 1):
+                call(side, forms[side], got[side][k], streams[side])
+    torch.cuda.synchronize()
+    for side in (0, 1):
+        for r in got[side]:
+            for k, x in alone[side].tensors.items():
+                assert torch.equal(x.view(torch.uint8),
+                                   r.tensors[k].view(torch.uint8)), (side, k)
