@@ -688,8 +688,17 @@ dprop_status launch(const dprop_config& c, const dprop_launch* launch_cfg,
     if (n == 0) {
         return DPROP_OK;
     }
+    // Work captured into the caller's graph is not staged: the capture would
+    // need an allocation when the kept area is too small, and its replays
+    // would share the area with calls it is not ordered against.
+    const bool use_graph = launch_cfg && launch_cfg->use_graph;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    DPROP_CUDA(cudaStreamIsCapturing(stream, &capture));
+    const bool no_stage =
+        !use_graph && capture != cudaStreamCaptureStatusNone;
     launch_plan plan = plan_launch(c, launch_cfg, det, field, io, n,
-                                   launch_cfg && launch_cfg->sort_tracks);
+                                   launch_cfg && launch_cfg->sort_tracks,
+                                   no_stage ? 0u : k_stage_limit);
     const uint32_t rec_cap =
         dprop::api::staged_capacity(make_prop_cfg<float>(c), io);
     const auto work_bytes = [&]() -> size_t {
@@ -697,7 +706,7 @@ dprop_status launch(const dprop_config& c, const dprop_launch* launch_cfg,
                                                               rec_cap)
                            : stage_bytes(n, plan.stage_cap);
     };
-    if (!(launch_cfg && launch_cfg->use_graph)) {
+    if (!use_graph) {
         launch_scratch scr{};
         dprop::api::kept_scratch::use sort_use, work_use;
         if (plan.sort) {
