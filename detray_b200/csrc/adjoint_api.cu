@@ -256,7 +256,7 @@ dprop_status dprop_propagate_adjoint(const dprop_config* cfg,
                 g_adj_sort.buf = nullptr;
                 g_adj_sort.bytes = 0;
             }
-            DPROP_CUDA(cudaMalloc(&g_adj_sort.buf, need));
+            DPROP_CUDA(api::alloc_device(&g_adj_sort.buf, need));
             g_adj_sort.bytes = need;
             g_adj_sort.device = dev;
         }

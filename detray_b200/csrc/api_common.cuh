@@ -38,6 +38,9 @@ class kept_scratch {
     };
 
 public:
+    // spare: given back when an allocation here finds no memory
+    explicit kept_scratch(kept_scratch* spare = nullptr) : spare_(spare) {}
+
     class use {
     public:
         use() = default;
@@ -59,12 +62,19 @@ public:
     cudaError_t take(size_t bytes, cudaStream_t stream, use* u);
     // Frees the buffers of all devices.
     void release();
+    // Frees the current device's buffer; whether there was one.
+    bool give_back();
 
 private:
+    kept_scratch* spare_;
     std::mutex mutex_;
     std::vector<slot> slots_;      // by device
     std::vector<void*> retired_;   // outgrown, but in a captured graph
 };
+
+// cudaMalloc; without room for it the staging area of sorted propagations, an
+// option that is kept between calls, is given back first.
+cudaError_t alloc_device(void** p, size_t bytes);
 
 // Number of a new detector or field handle, never given twice: a cached
 // CUDA graph is matched by it, since the address of a destroyed handle may be

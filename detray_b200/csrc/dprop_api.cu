@@ -84,7 +84,12 @@ cudaError_t kept_scratch::take(size_t bytes, cudaStream_t stream, use* u) {
         s.buf = nullptr;
         s.bytes = 0;
         s.captured = false;
-        if ((e = cudaMalloc(&s.buf, bytes)) != cudaSuccess) {
+        e = cudaMalloc(&s.buf, bytes);
+        if (e == cudaErrorMemoryAllocation && spare_ && spare_->give_back()) {
+            cudaGetLastError();
+            e = cudaMalloc(&s.buf, bytes);
+        }
+        if (e != cudaSuccess) {
             s.buf = nullptr;
             cudaGetLastError();
             return e;
@@ -126,6 +131,24 @@ void kept_scratch::release() {
     retired_.clear();
 }
 
+bool kept_scratch::give_back() {
+    std::lock_guard<std::mutex> lock(mutex_);
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        slots_.size() <= static_cast<size_t>(dev)) {
+        return false;
+    }
+    slot& s = slots_[static_cast<size_t>(dev)];
+    if (!s.buf || s.captured ||
+        (s.last && cudaEventSynchronize(s.last) != cudaSuccess)) {
+        return false;
+    }
+    cudaFree(s.buf);
+    s.buf = nullptr;
+    s.bytes = 0;
+    return true;
+}
+
 dprop_status cuda_fail(cudaError_t e, const char* what) {
     g_last_error = std::string(what) + ": " + cudaGetErrorString(e);
     return (e == cudaErrorMemoryAllocation) ? DPROP_E_OOM : DPROP_E_CUDA;
@@ -144,7 +167,8 @@ dprop_status upload(const std::vector<T>& h, T** d) {
     if (h.empty()) {
         return DPROP_OK;
     }
-    DPROP_CUDA(cudaMalloc(reinterpret_cast<void**>(d), h.size() * sizeof(T)));
+    DPROP_CUDA(dprop::api::alloc_device(reinterpret_cast<void**>(d),
+                                        h.size() * sizeof(T)));
     DPROP_CUDA(cudaMemcpy(*d, h.data(), h.size() * sizeof(T),
                           cudaMemcpyHostToDevice));
     return DPROP_OK;
@@ -172,17 +196,34 @@ dprop_status ensure_scratch(size_t bytes) {
         g_scratch.buf = nullptr;
         g_scratch.bytes = 0;
     }
-    DPROP_CUDA(cudaMalloc(&g_scratch.buf, bytes));
+    DPROP_CUDA(dprop::api::alloc_device(&g_scratch.buf, bytes));
     g_scratch.bytes = bytes;
     return DPROP_OK;
 }
 
-// Kept between calls: the direction sort's scratch, the slots and queues of the
-// persistent method, the staged results of sorted plain propagations.  A call
-// that needs two of them takes them in this order.
-dprop::api::kept_scratch g_sort;
-dprop::api::kept_scratch g_rounds;
+// Kept between calls: the staged results of sorted plain propagations, the
+// direction sort's scratch, the slots and queues of the persistent method.  A
+// call that needs two takes the sort's first, the staging area last.
 dprop::api::kept_scratch g_stage;
+dprop::api::kept_scratch g_sort{&g_stage};
+dprop::api::kept_scratch g_rounds{&g_stage};
+
+}  // namespace
+
+namespace dprop::api {
+
+cudaError_t alloc_device(void** p, size_t bytes) {
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation && g_stage.give_back()) {
+        cudaGetLastError();
+        e = cudaMalloc(p, bytes);
+    }
+    return e;
+}
+
+}  // namespace dprop::api
+
+namespace {
 
 // Sort key of a track, 20 bits: 7 bits of theta (major), 8 bits of phi, the
 // charge sign and 4 bits of log10(pT / GeV) over [-1, 2].  Tracks that share
@@ -769,8 +810,8 @@ dprop_status launch(const dprop_config& c, const dprop_launch* launch_cfg,
     // the next 256-byte boundary (an atomic on an unaligned word is a device
     // fault).
     const size_t rounds_offset = (sort_bytes + 255) & ~size_t(255);
-    cudaError_t me =
-        cudaMalloc(&e.scratch, rounds_offset + rounds_bytes + 256);
+    cudaError_t me = dprop::api::alloc_device(
+        &e.scratch, rounds_offset + rounds_bytes + 256);
     if (me == cudaErrorMemoryAllocation && plan.stage_cap > 0u) {
         cudaGetLastError();
         plan.stage_cap = 0u;
@@ -960,7 +1001,7 @@ dprop_status ensure_pipe(pipe_slot& ps, int index, size_t dev_bytes,
             ps.dev = nullptr;
             ps.dev_bytes = 0;
         }
-        DPROP_CUDA(cudaMalloc(&ps.dev, dev_bytes));
+        DPROP_CUDA(dprop::api::alloc_device(&ps.dev, dev_bytes));
         ps.dev_bytes = dev_bytes;
     }
     if (ps.host_entries < chunk + 1) {
@@ -1482,7 +1523,8 @@ dprop_status dprop_autotune(const dprop_config* cfg, const dprop_detector* det,
     const size_t per_track = 1 + 6 * 4 + 8 * 4 + 16;
     const size_t per_rec = 8 + 6 * 4 + 21 * 4 + 4 + 1;
     void* buf = nullptr;
-    DPROP_CUDA(cudaMalloc(&buf, m * per_track + cap * m * per_rec + 4096));
+    DPROP_CUDA(dprop::api::alloc_device(
+        &buf, m * per_track + cap * m * per_rec + 4096));
     char* p = static_cast<char*>(buf);
     auto take = [&](size_t b) {
         char* r = p;

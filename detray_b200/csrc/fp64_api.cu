@@ -96,7 +96,7 @@ dprop_status ensure_f64(f64_sort_scratch& sc, size_t need,
             sc.buf = nullptr;
             sc.bytes = 0;
         }
-        DPROP_CUDA(cudaMalloc(&sc.buf, need));
+        DPROP_CUDA(api::alloc_device(&sc.buf, need));
         sc.bytes = need;
         sc.device = dev;
     }

@@ -1,0 +1,63 @@
+"""Device memory the library keeps between calls: what is optional gives way
+to what a call needs."""
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+GB = 1 << 30
+
+
+@pytest.fixture
+def setup():
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from detray_b200 import geometry, propagator
+    from detray_b200.units import T
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    propagator.release_cache()
+    det = propagator.Detector(geometry.load_geometry("toy_4brl_7edc"))
+    field = propagator.Field.constant((0.0, 0.0, 2.0 * T))
+    yield torch, det, field
+    propagator.release_cache()
+    torch.cuda.empty_cache()
+
+
+def _device_tracks(torch, n, seed):
+    from detray_b200 import tracks
+    return torch.tensor(tracks.toy_tracks(n, seed=seed), dtype=torch.float32,
+                        device="cuda")
+
+
+def _fill(torch, leave):
+    """Take all device memory but ``leave`` bytes."""
+    free, _ = torch.cuda.mem_get_info()
+    return torch.empty(free - leave, dtype=torch.uint8, device="cuda")
+
+
+def test_staging_area_gives_way(setup):
+    """A persistent call whose slots fit only where a sorted plain call left
+    its staging area (300 000 x 32 records of 128 bytes: 1.2 GB)."""
+    torch, det, field = setup
+    from detray_b200 import abi, propagator
+    cfg = abi.make_config(max_records=32, search_window=(3, 3))
+    trk = _device_tracks(torch, 300000, 41)
+    res = propagator.alloc_device_results(300000, 32, "cuda")
+    few = trk[:, :150000].contiguous()
+    rounds = propagator.make_launch(method=abi.METHOD_PERSISTENT,
+                                    ctas_per_sm=3)
+    propagator.propagate(cfg, det, field, few, results=res, launch=rounds)
+    torch.cuda.synchronize()
+    want = res.tensors["n_steps"][:150000].clone()
+    propagator.release_cache()
+    propagator.propagate(cfg, det, field, trk, results=res,
+                         launch=propagator.make_launch(sort_tracks=1))
+    torch.cuda.synchronize()
+    # the slots and staged rows take 0.7 GB
+    filled = _fill(torch, GB // 2)
+    res.tensors["n_steps"].zero_()
+    propagator.propagate(cfg, det, field, few, results=res, launch=rounds)
+    torch.cuda.synchronize()
+    del filled
+    assert torch.equal(res.tensors["n_steps"][:150000], want)
