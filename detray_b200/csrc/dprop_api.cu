@@ -1134,21 +1134,38 @@ dprop_status propagate_host_jagged(const dprop_config& c,
     io_ptrs<double> any{};
     uint64_t some = 0u;
     any.rec_barcode = &some;
-    const launch_plan plan =
+    launch_plan plan =
         plan_launch(c, lc, det, field, any, chunk,
                     (lc == nullptr) || lc->sort_tracks != 0u,
                     k_stage_limit_host);
-    const size_t rounds_bytes =
+    size_t rounds_bytes =
         al256(plan.rounds ? dprop::api::rounds_scratch_bytes(
                                 chunk, det->wires, static_cast<uint32_t>(cap))
                           : stage_bytes(chunk, plan.stage_cap));
-    need += rounds_bytes;
-    for (int k = 0; k < n_slots; ++k) {
-        const dprop_status s = ensure_pipe(g_pipe[k], k, need, chunk);
-        if (s != DPROP_OK) {
-            return s;
+    dprop_status es = DPROP_OK;
+    for (int k = 0; k < n_slots && es == DPROP_OK; ++k) {
+        es = ensure_pipe(g_pipe[k], k, need + rounds_bytes, chunk);
+    }
+    if (es == DPROP_E_OOM && plan.stage_cap > 0u) {
+        // staging is an option: without room for it the chunks write their
+        // results directly
+        cudaGetLastError();
+        plan.stage_cap = 0u;
+        rounds_bytes = 0;
+        for (pipe_slot& ps : g_pipe) {
+            cudaFree(ps.dev);
+            ps.dev = nullptr;
+            ps.dev_bytes = 0;
+        }
+        es = DPROP_OK;
+        for (int k = 0; k < n_slots && es == DPROP_OK; ++k) {
+            es = ensure_pipe(g_pipe[k], k, need, chunk);
         }
     }
+    if (es != DPROP_OK) {
+        return es;
+    }
+    need += rounds_bytes;
     auto carve = [&](int sl) {
         return carve_slot(g_pipe[sl].dev, chunk, rec_slot, with_cov, sort_temp,
                           scan_temp);

@@ -61,3 +61,32 @@ def test_staging_area_gives_way(setup):
     torch.cuda.synchronize()
     del filled
     assert torch.equal(res.tensors["n_steps"][:150000], want)
+
+
+def test_host_pipeline_without_room_for_staging(setup):
+    """Jagged host call of 120 000 tracks, 64 records each: four chunks of
+    32 768 take 0.51 GB each, 0.78 GB with staging."""
+    torch, det, field = setup
+    import numpy as np
+    from detray_b200 import abi, propagator, tracks
+    cfg = abi.make_config(max_records=64, search_window=(3, 3))
+    trk = tracks.toy_tracks(120000, seed=42)
+    launch = propagator.make_launch(sort_tracks=1)
+
+    def run():
+        return propagator.propagate_host(cfg, det, field, trk, launch=launch,
+                                         jagged=True)
+
+    want = run()
+    propagator.release_cache()
+    filled = _fill(torch, int(2.5 * GB))
+    got = run()
+    del filled
+    total = int(want["rec_offsets"][-1])
+    assert total == int(got["rec_offsets"][-1])
+    for k in ("status", "n_records", "n_steps", "rec_offsets"):
+        assert np.array_equal(want[k], got[k]), k
+    assert np.array_equal(want["rec_barcode"][:total],
+                          got["rec_barcode"][:total])
+    assert np.array_equal(want["rec_bound"][:, :total].view(np.uint32),
+                          got["rec_bound"][:, :total].view(np.uint32))
