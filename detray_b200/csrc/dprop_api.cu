@@ -683,6 +683,7 @@ struct graph_entry {
     uint64_t field_id{0};
     cudaGraphExec_t exec{nullptr};
     void* scratch{nullptr};
+    size_t staged{0};  // bytes of the scratch that stage results
     uint64_t last_use{0};
     int device{0};
 };
@@ -803,6 +804,14 @@ dprop_status launch(const dprop_config& c, const dprop_launch* launch_cfg,
     e.det_id = det->id;
     e.field_id = field->id;
     e.device = dev;
+    // the graphs' staging areas together stay within the limit of one call
+    size_t staged = stage_bytes(n, plan.stage_cap);
+    for (const graph_entry& g : g_graphs) {
+        staged += g.device == dev ? g.staged : 0u;
+    }
+    if (staged > k_stage_limit) {
+        plan.stage_cap = 0u;
+    }
     const size_t sort_bytes = plan.sort ? sort_scratch_bytes(n) : 0;
     size_t rounds_bytes = work_bytes();
     // The radix sort's temporary size carries the sort's alignment padding
@@ -819,6 +828,7 @@ dprop_status launch(const dprop_config& c, const dprop_launch* launch_cfg,
         me = cudaMalloc(&e.scratch, rounds_offset + 256);
     }
     DPROP_CUDA(me);
+    e.staged = stage_bytes(n, plan.stage_cap);
     launch_scratch scr{};
     scr.sort = e.scratch;
     scr.sort_bytes = sort_bytes;

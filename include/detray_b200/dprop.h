@@ -605,8 +605,11 @@ dprop_status dprop_autotune(const dprop_config* cfg, const dprop_detector* det,
 
 /* Frees the device memory the library keeps between calls: the cached CUDA
  * graphs (use_graph) with the scratch each owns, and the grow-only scratch
- * of the direction sort, the persistent method and the host-buffer entry
- * points.  Synchronises the current device first; no propagate call may be
+ * of the direction sort, the persistent method, the staged results of sorted
+ * plain calls (max_records x 128 bytes per track, at most 8 GiB per device,
+ * at most 8 GiB in all cached graphs together, at most 2 GiB in each of the
+ * host pipeline's four slots) and the host-buffer entry points.  Staging is
+ * left out, or given back, where there is no memory for it.  Synchronises the current device first; no propagate call may be
  * running on another host thread.  Later calls allocate again on demand.
  * Counterpart of releasing the vecmem buffers the reference's caller owns. */
 dprop_status dprop_release_cache(void);

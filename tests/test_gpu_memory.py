@@ -36,7 +36,8 @@ def _fill(torch, leave):
     return torch.empty(free - leave, dtype=torch.uint8, device="cuda")
 
 
-def test_staging_area_gives_way(setup):
+@pytest.mark.parametrize("graph", [0, 1])
+def test_staging_area_gives_way(setup, graph):
     """A persistent call whose slots fit only where a sorted plain call left
     its staging area (300 000 x 32 records of 128 bytes: 1.2 GB)."""
     torch, det, field = setup
@@ -46,7 +47,7 @@ def test_staging_area_gives_way(setup):
     res = propagator.alloc_device_results(300000, 32, "cuda")
     few = trk[:, :150000].contiguous()
     rounds = propagator.make_launch(method=abi.METHOD_PERSISTENT,
-                                    ctas_per_sm=3)
+                                    ctas_per_sm=3, use_graph=graph)
     propagator.propagate(cfg, det, field, few, results=res, launch=rounds)
     torch.cuda.synchronize()
     want = res.tensors["n_steps"][:150000].clone()
@@ -90,3 +91,31 @@ def test_host_pipeline_without_room_for_staging(setup):
                           got["rec_barcode"][:total])
     assert np.array_equal(want["rec_bound"][:, :total].view(np.uint32),
                           got["rec_bound"][:, :total].view(np.uint32))
+
+
+def test_graphs_share_a_bound_on_staging(setup):
+    """Cached graphs of sorted plain calls own their staging areas (here 3.1 GB
+    each): together they hold at most 8 GiB, the next ones write directly."""
+    torch, det, field = setup
+    from detray_b200 import abi, propagator
+    cfg = abi.make_config(max_records=24, search_window=(3, 3))
+    n = 1000000
+    trk = _device_tracks(torch, n, 43)
+    launch = propagator.make_launch(sort_tracks=1, use_graph=1)
+    res = propagator.alloc_device_results(n, 24, "cuda")
+    torch.cuda.synchronize()
+    free, _ = torch.cuda.mem_get_info()
+    steps = []
+    for k in range(4):
+        # another number of tracks is another graph
+        m = n - 32 * k
+        sub = trk[:, :m].contiguous()
+        propagator.propagate(cfg, det, field, sub, results=res, launch=launch)
+        torch.cuda.synchronize()
+        steps.append(res.tensors["n_steps"][:n - 96].clone())
+        del sub
+    torch.cuda.empty_cache()
+    left, _ = torch.cuda.mem_get_info()
+    assert free - left < 9 * GB
+    for s in steps[1:]:
+        assert torch.equal(s, steps[0])
