@@ -223,15 +223,8 @@ dprop_status dprop_propagate_adjoint(const dprop_config* cfg,
     DPROP_CUDA(cudaGetDevice(&dev));
     DPROP_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     const uint64_t per_sm = n / static_cast<uint64_t>(sms);
-    // A warp per track pays for fewer tracks than in the normal propagation:
-    // the Jacobians, which the lanes repeat, are a larger part of a track.
-    // B200, us, against one thread per track: field gradient 1 000: 1 206 /
-    // 1 835, 2 000: 1 809 / 1 835, 3 000: 2 465 / 1 840; without 3 000: 1 256 /
-    // 1 685, 6 144: 2 154 / 1 690.
-    const uint64_t few = pc.step.field_gradient
-                             ? api::group_limit(det) / 4u
-                             : 2u * api::group_limit(det) / 3u;
-    if (api::open_shape(lc) && n <= few) {
+    if (api::open_shape(lc) &&
+        n <= group_limit_adjoint(det->traits, pc.step.field_gradient)) {
         if (!pc.step.field_gradient) {
             launch_adjoint_group<16, false>(st, det, field->view, pc, io, tv,
                                             n);

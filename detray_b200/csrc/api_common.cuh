@@ -10,6 +10,7 @@
 #include <string>
 #include <vector>
 
+#include "core/launch_rules.hpp"
 #include "core/propagate.cuh"
 #include "detray_b200/dprop.h"
 
@@ -133,6 +134,7 @@ struct dprop_detector {
     // material maps or volume material: launches use the kernels that
     // include the code for them
     bool wires{false};
+    dprop::launch_traits traits;
     dprop::detector_view<double> view_d() const { return view_d_as<true>(); }
     template <bool W>
     dprop::detector_view<double, W> view_d_as() const {

@@ -1,0 +1,132 @@
+// Which form a call takes that leaves its launch shape open: the properties of
+// a detector the rules look at, and the batch sizes where one form becomes
+// the faster one.  Every line holds both sides as measured (B200, 148 SMs,
+// microseconds, device time).
+#pragma once
+
+#include <cstdint>
+
+#include "detray_b200/dprop.h"
+
+namespace dprop {
+
+// What of a detector decides the form: not whether its kernels carry the code
+// for lines, rods, material maps and volume material (that is one flag for all
+// of them), but what a track spends its time on.
+struct launch_traits {
+    bool lines{false};          // line surfaces or several surfaces per bin:
+                                // long tracks, many candidates a volume
+    bool surface_grids{false};  // volumes find their surfaces in grids
+    bool extra_code{false};     // kernels with the code of all options (a
+                                // lone warp waits longer for instructions)
+};
+
+inline launch_traits launch_traits_of(const dprop_detector_desc* d,
+                                      bool extra_code) {
+    launch_traits t;
+    t.extra_code = extra_code;
+    for (uint32_t i = 0; i < d->n_surfaces; ++i) {
+        t.lines = t.lines || d->surfaces[i].shape == DPROP_SHAPE_LINE;
+    }
+    for (uint32_t i = 0; i < d->n_volumes; ++i) {
+        const uint32_t g = d->volumes[i].grid;
+        if (g != DPROP_INVALID_INDEX) {
+            t.surface_grids = true;
+            t.lines = t.lines || d->grids[g].multi != 0u;
+        }
+    }
+    return t;
+}
+
+// Tracks up to which a warp per track is the faster form, fp32.  The lanes of a
+// warp share only the searches, so beyond a full GPU one thread per track
+// wins; how far beyond depends on how much of a track is search.  Warp per
+// track / thread per track in input order / sorted:
+//   toy 5 000: 1 025 / 1 882 / 1 356, 8 000: 1 566 / 1 910 / 1 381; in the map
+//   5 000: 1 218 / 1 956 / 1 418
+//   toy with material maps 4 000: 1 658 / 2 002 / 1 575, 5 000: 1 979 / 2 035 /
+//   1 616, 10 000: 3 954 / 2 017 / 1 566
+//   wire chamber, pT from 0.5 GeV, |eta| < 1, 5 000: 1 939 / 2 361 / 2 517,
+//   8 000: 2 814 / 2 399 / 2 511; pT from 0.1 GeV, |eta| < 3, 8 000: 4 134 /
+//   7 577 / 10 225
+//   telescope (no grid, 11 surfaces) 2 300: 215 / 249 / 307, 3 000: 340 / 248 /
+//   308; with volume material 1 400: 305 / 322 / 384, 1 800: 328 / 316 / 389,
+//   10 000: 1 669 / 347 / 430
+inline uint64_t group_limit(const launch_traits& t) {
+    if (t.lines) {
+        return 8192u;
+    }
+    if (t.surface_grids) {
+        return t.extra_code ? 4096u : 6144u;
+    }
+    return t.extra_code ? 1536u : 2368u;
+}
+
+// The same in the adjoint propagation.  It pays for fewer tracks there: the
+// Jacobians, which the lanes repeat, are a larger part of a track.  Warp per
+// track / thread per track / sorted, with the field gradient:
+//   toy in the map 1 400: 1 434 / 2 187 / 1 696, 1 800: 1 480 / 2 151 / 1 641;
+//   with material maps 1 000: 1 648 / 2 409 / 1 927, 1 400: 2 289 / 2 455 /
+//   1 940; wire chamber 2 300: 2 891 / 3 028 / 3 050, 3 000: 4 060 / 3 107 /
+//   3 102; telescope 700: 492 / 519 / 572, 1 400: 655 / 525 / 584
+// and without it:
+//   toy 4 000: 1 368 / 2 067 / 1 585, 5 000: 1 659 / 2 125 / 1 585; with
+//   material maps 2 300: 1 491 / 2 403 / 1 835, 3 000: 2 051 / 2 425 / 1 774;
+//   wire chamber 5 000: 3 100 / 2 799 / 2 962 (pT from 0.1 GeV 3 843 / 8 274 /
+//   8 223); telescope 1 400: 345 / 384 / 455, 3 000: 537 / 396 / 472
+inline uint64_t group_limit_adjoint(const launch_traits& t,
+                                    bool field_gradient) {
+    return field_gradient ? group_limit(t) / 4u : 2u * group_limit(t) / 3u;
+}
+
+// The same in double precision.  Warp per track / thread per track / sorted:
+// toy 3 000: 1 255 / 1 763 / 1 307, 4 000: 1 575 / 1 729 / 1 347; with material
+// maps 2 300: 1 761 / 2 455 / 1 827, 3 000: 2 406 / 2 440 / 1 775, 8 000: 6 426 /
+// 2 501 / 1 889; wire chamber 4 000: 2 969 / 2 840 / 2 879, 5 000: 3 649 / 2 891 /
+// 2 972 (pT from 0.1 GeV 4 640 / 8 960 / 8 862); telescope 1 000: 217 / 288 /
+// 355, 1 800: 333 / 289 / 353; with volume material 1 000: 326 / 411 / 478,
+// 1 400: 529 / 425 / 483, 8 000: 2 206 / 436 / 527.
+inline uint64_t group_limit_fp64(const launch_traits& t) {
+    if (t.lines) {
+        return 5120u;
+    }
+    if (t.surface_grids) {
+        return 3072u;
+    }
+    return t.extra_code ? 1184u : 2048u;
+}
+
+// Tracks from which the round-based method is the faster form of a call that
+// asks for it: below, its rounds' latency (some 50 of 80 us) outweighs the
+// plain kernel's divergence.  Plain sorted / rounds:
+//   toy 200 000: 5 622 / 6 075, 400 000: 9 129 / 9 080, 1 000 000: 21 051 /
+//   18 001; in the map 150 000: 6 096 / 6 118, 250 000: 9 962 / 7 903
+//   toy with material maps 120 000: 5 061 / 6 342, 230 000: 9 663 / 9 639,
+//   300 000: 11 057 / 10 229; in the map 120 000: 5 730 / 6 680, 230 000:
+//   10 371 / 9 269
+//   wire chamber, pT from 0.1 GeV, 12 289: 9 587 / 11 104, 20 000: 11 782 /
+//   11 692; from 0.5 GeV 30 000: 3 763 / 4 376, 60 000: 5 228 / 4 682
+//   a telescope without surface grids 1 000 000: 5 349 / 6 168, with volume
+//   material 8 135 / 8 473
+inline uint64_t rounds_from(const launch_traits& t, bool field_map) {
+    if (t.lines) {
+        return 16384u;
+    }
+    if (!t.surface_grids) {
+        return ~uint64_t(0);
+    }
+    if (field_map) {
+        return 150000u;
+    }
+    return t.extra_code ? 230000u : 400000u;
+}
+
+// The same in double precision: toy in the map 75 000: 5 785 / 6 651, 100 000:
+// 9 351 / 7 264; constant field 75 000: 3 544 / 5 817, 100 000: 5 679 / 6 314;
+// with material maps 40 000: 4 396 / 6 300, 80 000: 7 953 / 7 096; wire chamber,
+// pT from 0.1 GeV, 16 000: 12 835 / 13 846, 30 000: 16 817 / 14 452.
+inline uint64_t rounds_from_fp64(const launch_traits& t) {
+    return t.lines ? 25000u : 80000u;
+}
+
+}  // namespace dprop

@@ -579,23 +579,6 @@ struct launch_plan {
     uint32_t stage_cap{0};  // plain: records per track staged (0: none)
 };
 
-// Tracks from which the round-based method is the faster form of a call that
-// asks for it and leaves the shape open: below, its rounds' latency (some 50
-// of 80 us) outweighs the plain kernel's divergence.  B200, us, plain sorted
-// against rounds: toy 200 000: 5 622 / 6 075, 400 000: 9 129 / 9 080,
-// 1 000 000: 21 051 / 18 001; in the field map 150 000: 6 096 / 6 118,
-// 250 000: 9 962 / 7 903; wire chamber 12 289: 9 587 / 11 104, 20 000: 11 782 /
-// 11 692; a telescope without surface grids 1 000 000: 5 349 / 6 168.
-uint64_t rounds_from(const dprop_detector* det, const dprop_field* field) {
-    if (det->wires) {
-        return 16384u;
-    }
-    if (det->grids == nullptr) {
-        return ~uint64_t(0);
-    }
-    return field->view.kind == 0u ? 400000u : 150000u;
-}
-
 // Tracks from which the results of a sorted plain propagation are staged: a
 // sorted track's record, written field by field at its input index, touches
 // 31 sectors for 121 bytes.  Smaller batches stay in L2, which merges them.
@@ -621,7 +604,8 @@ launch_plan plan_launch(const dprop_config& c, const dprop_launch* lc,
     }
     const bool open = dprop::api::open_shape(lc) && !fg;
     p.rounds = lc && lc->method == DPROP_METHOD_PERSISTENT &&
-               !(open && n < rounds_from(det, field));
+               !(open &&
+                 n < rounds_from(det->traits, field->view.kind != 0u));
     const bool staged = io.rec_barcode != nullptr && n >= k_stage_from &&
                         stage_bytes(n, c.max_records) <= stage_limit;
     // without surface grids every track tests the same few surfaces: an order
@@ -1489,6 +1473,7 @@ dprop_status dprop_detector_create(const dprop_detector_desc* d, int device,
     for (uint32_t i = 0; i < d->n_grids; ++i) {
         det->wires = det->wires || d->grids[i].multi != 0u;
     }
+    det->traits = launch_traits_of(d, det->wires);
     const host_tables<double> td = convert_desc<double>(d);
     if ((st = upload(td.nav_surfaces, &det->nav_surfaces_d)) != DPROP_OK ||
         (st = upload(td.masks, &det->masks_d)) != DPROP_OK ||

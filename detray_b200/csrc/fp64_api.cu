@@ -27,25 +27,6 @@ namespace {
 
 constexpr int k_f64_block = 128;
 
-// The forms of a call that leaves its shape open, by batch size (B200, us).
-// A warp per track against one thread per track: toy in the field map 1 000:
-// 727 / 2 157, 4 000: 2 049 / 2 190 (2 051 sorted), constant field 4 000: 1 485
-// / 1 661 (1 204 sorted); wire chamber 4 000: 5 623 / 9 391, 8 000: 9 265 /
-// 10 826.
-uint64_t f64_group_limit(const dprop_detector* det) {
-    if (det->wires) {
-        return 8192u;
-    }
-    return det->grids != nullptr ? 3072u : 2048u;
-}
-// Plain (sorted) against the round-based method: toy in the map 75 000:
-// 5 785 / 6 651, 100 000: 9 351 / 7 264; constant field 75 000: 3 544 / 5 817,
-// 100 000: 5 679 / 6 314; wire chamber 16 000: 12 835 / 13 846, 30 000: 16 817 /
-// 14 452.
-uint64_t f64_rounds_from(const dprop_detector* det) {
-    return det->wires ? 25000u : 80000u;
-}
-
 template <int MinBlocks, bool W, bool Grad = false>
 __global__ void __launch_bounds__(k_f64_block, MinBlocks)
     propagate_fp64_kernel(const __grid_constant__ detector_view<double, W> det,
@@ -122,7 +103,7 @@ dprop_status propagate_fp64(const dprop_config& c, const dprop_launch* lc,
     DPROP_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     const uint64_t per_sm = n / static_cast<uint64_t>(sms);
     const bool open = open_shape(lc) && c.use_field_gradient == 0;
-    if (open && n <= f64_group_limit(det)) {
+    if (open && n <= group_limit_fp64(det->traits)) {
         auto go = [&](auto view) {
             constexpr bool W =
                 std::is_same<decltype(view), detector_view<double, true>>::value;
@@ -159,7 +140,7 @@ dprop_status propagate_fp64(const dprop_config& c, const dprop_launch* lc,
         }
     }
     if (lc && lc->method == DPROP_METHOD_PERSISTENT &&
-        !(open && n < f64_rounds_from(det))) {
+        !(open && n < rounds_from_fp64(det->traits))) {
         const size_t need = rounds_scratch_bytes_fp64(
             n, det->wires, staged_capacity(pc, io));
         const dprop_status e = ensure_f64(g_f64_rounds, need, stream);

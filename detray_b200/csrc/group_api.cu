@@ -49,20 +49,6 @@ void launch_group(cudaStream_t st, const dprop_detector* det,
 
 namespace dprop::api {
 
-// Tracks up to which a warp per track is the faster form.  The lanes of a
-// warp share only the searches, so beyond a full GPU one thread per track
-// wins; how far beyond depends on how much of a track is search.  Measured
-// (B200, warp per track against thread per track, us): toy detector 5 000:
-// 1 265 / 2 073 (1 545 direction-sorted), 10 000: 2 531 / 2 156; wire chamber
-// 10 000: 7 027 / 11 652, 20 000: 12 288 / 13 890; a telescope (no surface
-// grid, 11 surfaces) 1 000: 172 / 303, 3 000: 342 / 310.
-uint64_t group_limit(const dprop_detector* det) {
-    if (det->wires) {
-        return 12288u;
-    }
-    return det->grids != nullptr ? 6144u : 2368u;
-}
-
 bool open_shape(const dprop_launch* lc) {
     return !lc || (lc->block_size | lc->ctas_per_sm | lc->steps_per_round |
                    lc->rounds | lc->yield_lanes | lc->sort_interval |
@@ -72,7 +58,7 @@ bool open_shape(const dprop_launch* lc) {
 bool use_group(const dprop_launch* lc, const dprop_detector* det,
                bool field_gradient, uint64_t n) {
     // a launch shape that is spelled out is launched as it is
-    return open_shape(lc) && !field_gradient && n <= group_limit(det);
+    return open_shape(lc) && !field_gradient && n <= group_limit(det->traits);
 }
 
 template <typename In>

@@ -246,8 +246,6 @@ __device__ __forceinline__ void run_group(uint64_t t, uint64_t n,
 // enqueue of that form (no scratch, no order: every track has its own warp).
 bool use_group(const dprop_launch* lc, const dprop_detector* det,
                bool field_gradient, uint64_t n);
-// Batch size up to which that is the faster form.
-uint64_t group_limit(const dprop_detector* det);
 // Whether the launch leaves its shape open (method and sort apart).
 bool open_shape(const dprop_launch* lc);
 template <typename In>

@@ -1,0 +1,22 @@
+// TEST-ONLY: the batch sizes at which an open launch shape changes its form.
+#include "core/convert.hpp"
+#include "core/launch_rules.hpp"
+
+using namespace dprop;
+
+// extra_code: as the library finds it (line surfaces, rods, multi-entry bins,
+// material maps, volume material)
+extern "C" int launch_rules(const dprop_detector_desc* d, int extra_code,
+                            int field_map, uint64_t* out) {
+    if (!validate_desc(d).empty()) {
+        return 1;
+    }
+    const launch_traits t = launch_traits_of(d, extra_code != 0);
+    out[0] = group_limit(t);
+    out[1] = group_limit_fp64(t);
+    out[2] = group_limit_adjoint(t, false);
+    out[3] = group_limit_adjoint(t, true);
+    out[4] = rounds_from(t, field_map != 0);
+    out[5] = rounds_from_fp64(t);
+    return 0;
+}

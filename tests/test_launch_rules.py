@@ -1,0 +1,84 @@
+"""The forms of an open launch shape follow what a track spends its time on,
+not which options its kernels are compiled with: a detector with material maps
+or volume material is no wire detector.  The bounds are batch sizes at which
+the other form was measured at least 1.2 times slower."""
+import ctypes as C
+import subprocess
+from pathlib import Path
+
+import numpy as np
+import pytest
+
+REPO = Path(__file__).resolve().parents[1]
+NEVER = 2**64 - 1
+
+
+@pytest.fixture(scope="module")
+def rules(tmp_path_factory):
+    from detray_b200 import abi, build, geometry
+    out = tmp_path_factory.mktemp("rules") / "librules.so"
+    inc = Path(build.nvcc()).resolve().parent.parent / "include"
+    subprocess.run(["g++", "-std=c++17", "-O1", "-fPIC", "-shared",
+                    f"-I{REPO / 'include'}", f"-I{build.CSRC}", f"-I{inc}",
+                    str(REPO / "tests" / "native" / "launch_rules.cpp"),
+                    "-o", str(out)], check=True)
+    lib = C.CDLL(str(out))
+
+    def get(tables, extra_code, field_map=0):
+        desc = geometry.Descriptor(tables)
+        v = (C.c_uint64 * 6)()
+        assert lib.launch_rules(C.byref(desc.desc), extra_code, field_map,
+                                v) == 0
+        return dict(zip(("group", "group64", "adjoint", "adjoint_grad",
+                         "rounds", "rounds64"), v))
+
+    get.load = geometry.load_geometry
+    get.abi = abi
+    return get
+
+
+def test_material_maps_are_no_wire_detector(rules):
+    toy = rules(rules.load("toy_4brl_7edc"), 0)
+    maps = rules(rules.load("toy_4brl_7edc_maps"), 1)
+    assert 3000 <= maps["group"] <= 5000 < toy["group"] <= 7000
+    assert maps["group64"] <= 3500
+    assert maps["adjoint"] <= 3000 and maps["adjoint_grad"] <= 1400
+    assert maps["rounds"] >= 120000 and maps["rounds64"] >= 40000
+    assert rules(rules.load("toy_4brl_7edc_maps"), 1, 1)["rounds"] >= 120000
+
+
+def test_volume_material_is_no_wire_detector(rules):
+    t = {k: v.copy() for k, v in rules.load("telescope_10x1m_300um").items()}
+    slabs = t["slabs"]
+    t["volumes"]["material"] = int(np.flatnonzero(
+        (slabs["X0"] > 0) & (slabs["mean_excitation_energy"] > 0))[0])
+    got = rules(t, 1)
+    assert got["group"] <= 1800 and got["group64"] <= 1400
+    assert got["rounds"] == NEVER
+
+
+def test_material_maps_are_no_surface_grids(rules):
+    """A telescope whose volumes have no grid, beside a grid that is a
+    material map."""
+    t = {k: v.copy() for k, v in rules.load("telescope_10x1m_300um").items()}
+    maps = rules.load("toy_4brl_7edc_maps")
+    abi = rules.abi
+    kinds = maps["grids"]["kind"]
+    i = int(np.flatnonzero(kinds >= 3)[0])
+    g = maps["grids"][i:i + 1].copy()
+    n = int(g["n_bins"][0][0] * g["n_bins"][0][1])
+    g["bin_offset"] = 0
+    g["transform"] = 0
+    t["grids"] = g
+    t["grid_bins"] = np.zeros(n, np.uint32)
+    assert (t["volumes"]["grid"] == abi.DPROP_INVALID_INDEX).all()
+    assert rules(t, 1)["rounds"] == NEVER
+
+
+def test_wire_chamber(rules):
+    for name in ("wire_chamber_10l_cells", "wire_chamber_10l_straws"):
+        got = rules(rules.load(name), 1)
+        assert 5000 <= got["group"] <= 8200
+        assert got["group64"] <= 6000
+        assert got["adjoint"] <= 5500 and got["adjoint_grad"] <= 2100
+        assert got["rounds"] <= 30000
