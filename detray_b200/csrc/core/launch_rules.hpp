@@ -106,14 +106,15 @@ inline uint64_t group_limit_fp64(const launch_traits& t) {
 //   10 371 / 9 269
 //   wire chamber, pT from 0.1 GeV, 12 289: 9 587 / 11 104, 20 000: 11 782 /
 //   11 692; from 0.5 GeV 30 000: 3 763 / 4 376, 60 000: 5 228 / 4 682
-//   a telescope without surface grids 1 000 000: 5 349 / 6 168, with volume
-//   material 8 135 / 8 473
+//   a telescope without surface grids 1 000 000: 5 349 / 6 168; with volume
+//   material 300 000: 2 476 / 3 454, 1 000 000: 8 135 / 8 473, in the map 9 235 /
+//   9 084
 inline uint64_t rounds_from(const launch_traits& t, bool field_map) {
     if (t.lines) {
         return 16384u;
     }
     if (!t.surface_grids) {
-        return ~uint64_t(0);
+        return t.extra_code ? 1000000u : ~uint64_t(0);
     }
     if (field_map) {
         return 150000u;
@@ -127,6 +128,29 @@ inline uint64_t rounds_from(const launch_traits& t, bool field_map) {
 // pT from 0.1 GeV, 16 000: 12 835 / 13 846, 30 000: 16 817 / 14 452.
 inline uint64_t rounds_from_fp64(const launch_traits& t) {
     return t.lines ? 25000u : 80000u;
+}
+
+// Register budget of the plain kernel, fp32: resident CTAs of 128 threads per
+// SM, 4 (128 registers) while that keeps the whole batch resident, 512 tracks
+// per SM; else 8 (64).  In a field map 16 (32 registers) from 1 536 per SM on
+// when the volumes have surface grids: more warps hide the lookups and the
+// grid's loads.  Tracks that test a list have less to hide.  4 / 8 / 12 / 16:
+//   toy 75 000: 2 532 / 2 742 / 3 210 / 3 526, 150 000: 4 847 / 3 710 / 4 770 /
+//   4 972, 1 200 000: - / 25 022 / 27 294 / 25 483; in the map 150 000: 7 772 /
+//   6 169 / 7 846 / 8 051, 300 000: - / 11 694 / 13 054 / 10 778
+//   wire chamber in the map 300 000: - / 19 504 / 23 051 / 17 542; toy with
+//   material maps in the map 300 000: - / 12 556 / 13 829 / 11 860
+//   telescope 10 000: 234 / 276 / 317 / 347; in the map 300 000: - / 2 051 /
+//   2 706 / 2 927, 1 000 000: - / 6 570 / 8 231 / 9 537
+//   the toy detector's modules as lists (1 096 in a volume), in the map, input
+//   order 230 000: 49 412 / 28 715 / 34 391 / 34 001, sorted 25 674 / 18 328 /
+//   18 072 / 22 662
+inline int plain_budget(const launch_traits& t, bool field_map,
+                        uint64_t tracks_per_sm) {
+    if (tracks_per_sm < 512u) {
+        return 4;
+    }
+    return field_map && t.surface_grids && tracks_per_sm >= 1536u ? 16 : 8;
 }
 
 }  // namespace dprop

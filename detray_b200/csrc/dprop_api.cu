@@ -475,16 +475,10 @@ int plain_block_of(const dprop_launch* lc) {
     return static_cast<int>(b);
 }
 
-// Register budget of a plain launch (resident CTAs of 128 threads per SM).
-// Left open: 4 (128 registers) while that keeps the whole batch resident, 512
-// tracks per SM; else 8 (64); in a field map from 1 536 tracks per SM on 16
-// (32), whose warps hide the lookups.  B200, us with 4 / 8 / 12 / 16: toy
-// 75 000: 2 532 / 2 742 / 3 210 / 3 526; 150 000: 4 847 / 3 710 / 4 770 /
-// 4 972; 1 200 000: - / 25 022 / 27 294 / 25 483; in the map 150 000: 7 772 /
-// 6 169 / 7 846 / 8 051, 300 000: - / 11 694 / 13 054 / 10 778; telescope
-// 10 000: 234 / 276 / 317 / 347.
-dprop_status plain_budget(const dprop_launch* lc, const field_view<float>& field,
-                          uint64_t n, int* mb) {
+// Register budget of a plain launch, the spelled-out one or plain_budget's.
+dprop_status launch_budget(const dprop_launch* lc, const dprop_detector* det,
+                           const field_view<float>& field, uint64_t n,
+                           int* mb) {
     *mb = occupancy_of(lc);
     if (lc && lc->ctas_per_sm) {
         return DPROP_OK;
@@ -492,8 +486,8 @@ dprop_status plain_budget(const dprop_launch* lc, const field_view<float>& field
     int dev = 0, sms = 0;
     DPROP_CUDA(cudaGetDevice(&dev));
     DPROP_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    const uint64_t per_sm = n / static_cast<uint64_t>(sms);
-    *mb = per_sm < 512u ? 4 : (field.kind != 0u && per_sm >= 1536u ? 16 : 8);
+    *mb = plain_budget(det->traits, field.kind != 0u,
+                       n / static_cast<uint64_t>(sms));
     return DPROP_OK;
 }
 
@@ -513,7 +507,7 @@ dprop_status launch_plain(const dprop_launch* lc, cudaStream_t st,
                     "256");
     }
     int mb = 0;
-    const dprop_status s = plain_budget(lc, field, n, &mb);
+    const dprop_status s = launch_budget(lc, det, field, n, &mb);
     if (s != DPROP_OK) {
         return s;
     }

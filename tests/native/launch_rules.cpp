@@ -6,6 +6,12 @@ using namespace dprop;
 
 // extra_code: as the library finds it (line surfaces, rods, multi-entry bins,
 // material maps, volume material)
+extern "C" int plain_budget_of(const dprop_detector_desc* d, int extra_code,
+                               int field_map, uint64_t tracks_per_sm) {
+    return plain_budget(launch_traits_of(d, extra_code != 0), field_map != 0,
+                        tracks_per_sm);
+}
+
 extern "C" int launch_rules(const dprop_detector_desc* d, int extra_code,
                             int field_map, uint64_t* out) {
     if (!validate_desc(d).empty()) {

@@ -32,6 +32,12 @@ def rules(tmp_path_factory):
         return dict(zip(("group", "group64", "adjoint", "adjoint_grad",
                          "rounds", "rounds64"), v))
 
+    def budget(tables, extra_code, field_map, tracks_per_sm):
+        desc = geometry.Descriptor(tables)
+        return lib.plain_budget_of(C.byref(desc.desc), extra_code, field_map,
+                                   C.c_uint64(tracks_per_sm))
+
+    get.budget = budget
     get.load = geometry.load_geometry
     get.abi = abi
     return get
@@ -54,7 +60,7 @@ def test_volume_material_is_no_wire_detector(rules):
         (slabs["X0"] > 0) & (slabs["mean_excitation_energy"] > 0))[0])
     got = rules(t, 1)
     assert got["group"] <= 1800 and got["group64"] <= 1400
-    assert got["rounds"] == NEVER
+    assert got["rounds"] >= 700000
 
 
 def test_material_maps_are_no_surface_grids(rules):
@@ -72,7 +78,11 @@ def test_material_maps_are_no_surface_grids(rules):
     t["grids"] = g
     t["grid_bins"] = np.zeros(n, np.uint32)
     assert (t["volumes"]["grid"] == abi.DPROP_INVALID_INDEX).all()
-    assert rules(t, 1)["rounds"] == NEVER
+    assert rules(t, 1)["rounds"] >= 700000
+
+
+def test_telescope(rules):
+    assert rules(rules.load("telescope_10x1m_300um"), 0)["rounds"] == NEVER
 
 
 def test_wire_chamber(rules):
@@ -82,3 +92,17 @@ def test_wire_chamber(rules):
         assert got["group64"] <= 6000
         assert got["adjoint"] <= 5500 and got["adjoint_grad"] <= 2100
         assert got["rounds"] <= 30000
+
+
+def test_budget_of_large_batches(rules):
+    """32 registers per thread pay in a field map where volumes have surface
+    grids, and only there."""
+    big = 2000
+    assert rules.budget(rules.load("toy_4brl_7edc"), 0, 1, big) == 16
+    assert rules.budget(rules.load("wire_chamber_10l_cells"), 1, 1, big) == 16
+    assert rules.budget(rules.load("toy_4brl_7edc"), 0, 0, big) == 8
+    tele = rules.load("telescope_10x1m_300um")
+    for extra in (0, 1):
+        for field_map in (0, 1):
+            assert rules.budget(tele, extra, field_map, big) == 8
+            assert rules.budget(tele, extra, field_map, 511) == 4
