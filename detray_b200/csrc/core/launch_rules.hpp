@@ -17,6 +17,8 @@ struct launch_traits {
     bool lines{false};          // line surfaces or several surfaces per bin:
                                 // long tracks, many candidates a volume
     bool surface_grids{false};  // volumes find their surfaces in grids
+    bool long_lists{false};     // more than 32 surfaces in a volume's
+                                // brute-force list
     bool extra_code{false};     // kernels with the code of all options (a
                                 // lone warp waits longer for instructions)
 };
@@ -29,6 +31,8 @@ inline launch_traits launch_traits_of(const dprop_detector_desc* d,
         t.lines = t.lines || d->surfaces[i].shape == DPROP_SHAPE_LINE;
     }
     for (uint32_t i = 0; i < d->n_volumes; ++i) {
+        t.long_lists = t.long_lists ||
+                       d->volumes[i].bf_end - d->volumes[i].bf_begin > 32u;
         const uint32_t g = d->volumes[i].grid;
         if (g != DPROP_INVALID_INDEX) {
             t.surface_grids = true;
@@ -128,6 +132,18 @@ inline uint64_t rounds_from(const launch_traits& t, bool field_map) {
 // pT from 0.1 GeV, 16 000: 12 835 / 13 846, 30 000: 16 817 / 14 452.
 inline uint64_t rounds_from_fp64(const launch_traits& t) {
     return t.lines ? 25000u : 80000u;
+}
+
+// Whether a plain propagation that asks for direction order is faster without
+// it: where every track tests the same few surfaces an order gains little and
+// scatters the results, unless they are staged or the batch is large.  Input
+// order / sorted, fp32:
+//   telescope (16 surfaces in the list) 10 000: 260 / 344, in the map 298 / 369;
+//   without records 20 000: 297 / 323, 40 000: 352 / 335, 300 000: 1 543 / 1 328
+//   the toy detector's modules as lists (1 096) 3 000: 14 098 / 12 685, 14 000:
+//   14 539 / 11 937, 300 000 without records: 31 888 / 18 061
+inline bool order_is_a_loss(const launch_traits& t, bool staged, uint64_t n) {
+    return !t.surface_grids && !t.long_lists && !staged && n < 32768u;
 }
 
 // Register budget of the plain kernel, fp32: resident CTAs of 128 threads per

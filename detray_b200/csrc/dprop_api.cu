@@ -602,10 +602,8 @@ launch_plan plan_launch(const dprop_config& c, const dprop_launch* lc,
                  n < rounds_from(det->traits, field->view.kind != 0u));
     const bool staged = io.rec_barcode != nullptr && n >= k_stage_from &&
                         stage_bytes(n, c.max_records) <= stage_limit;
-    // without surface grids every track tests the same few surfaces: an order
-    // gains little there and scatters the results (telescope, 10 000 tracks:
-    // 234 us in input order, 336 us sorted)
-    p.sort = sort && (p.rounds || !open || staged || det->grids != nullptr);
+    p.sort = sort && (p.rounds || !open ||
+                      !order_is_a_loss(det->traits, staged, n));
     if (!p.rounds && p.sort && staged) {
         p.stage_cap = c.max_records;
     }

@@ -12,6 +12,11 @@ extern "C" int plain_budget_of(const dprop_detector_desc* d, int extra_code,
                         tracks_per_sm);
 }
 
+extern "C" int drops_order(const dprop_detector_desc* d, int staged,
+                           uint64_t n) {
+    return order_is_a_loss(launch_traits_of(d, false), staged != 0, n) ? 1 : 0;
+}
+
 extern "C" int launch_rules(const dprop_detector_desc* d, int extra_code,
                             int field_map, uint64_t* out) {
     if (!validate_desc(d).empty()) {

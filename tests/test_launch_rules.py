@@ -37,7 +37,13 @@ def rules(tmp_path_factory):
         return lib.plain_budget_of(C.byref(desc.desc), extra_code, field_map,
                                    C.c_uint64(tracks_per_sm))
 
+    def drops_order(tables, staged, n):
+        desc = geometry.Descriptor(tables)
+        return bool(lib.drops_order(C.byref(desc.desc), staged,
+                                    C.c_uint64(n)))
+
     get.budget = budget
+    get.drops_order = drops_order
     get.load = geometry.load_geometry
     get.abi = abi
     return get
@@ -106,3 +112,37 @@ def test_budget_of_large_batches(rules):
         for field_map in (0, 1):
             assert rules.budget(tele, extra, field_map, big) == 8
             assert rules.budget(tele, extra, field_map, 511) == 4
+
+
+def _grids_as_lists(tables, abi):
+    """The surfaces of every volume's grid in its brute-force list."""
+    t = {k: v.copy() for k, v in tables.items()}
+    lists = []
+    for v in t["volumes"]:
+        own = list(t["bf_surfaces"][v["bf_begin"]:v["bf_end"]])
+        if v["grid"] != abi.DPROP_INVALID_INDEX:
+            g = t["grids"][v["grid"]]
+            n = int(g["n_bins"][0]) * int(g["n_bins"][1])
+            bins = t["grid_bins"][g["bin_offset"]:g["bin_offset"] + n]
+            own += sorted(set(bins[bins != abi.DPROP_INVALID_INDEX].tolist()))
+            v["grid"] = abi.DPROP_INVALID_INDEX
+        v["bf_begin"], v["bf_end"] = len(lists), len(lists) + len(own)
+        lists += own
+    t["bf_surfaces"] = np.array(lists, np.uint32)
+    t["grids"] = t["grids"][:0]
+    t["grid_bins"] = t["grid_bins"][:0]
+    return t
+
+
+def test_requested_order_is_kept(rules):
+    """A requested direction order is only left out for short lists, small
+    batches and direct results."""
+    tele = rules.load("telescope_10x1m_300um")
+    assert rules.drops_order(tele, 0, 10000)
+    assert not rules.drops_order(tele, 1, 20000)
+    assert not rules.drops_order(tele, 0, 40000)
+    toy = rules.load("toy_4brl_7edc")
+    assert not rules.drops_order(toy, 0, 10000)
+    lists = _grids_as_lists(toy, rules.abi)
+    for n in (3000, 14000, 300000):
+        assert not rules.drops_order(lists, 0, n)
