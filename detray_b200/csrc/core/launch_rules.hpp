@@ -134,6 +134,20 @@ inline uint64_t rounds_from_fp64(const launch_traits& t) {
     return t.lines ? 25000u : 80000u;
 }
 
+// Tracks left to the tail of the round-based method, below which it begins
+// when the launch does not say: n / 64, but no more than the kernel that runs
+// a warp per track takes.  Beyond, the tail ran one thread per track, whose
+// step is the slower one, and the longest track's steps are the tail's time.
+// Rounds with n / 64 / with the bound, ms: wire chamber in the map, 2 M tracks
+// from 0.1 GeV, one of them stepping 100 000 times 629 / 533, 200 / 178; toy
+// with material maps in the map, 1 M from 0.1 GeV 98.2 / 49.3; in double
+// precision 1 M toy tracks 55.1 / 46.5; 1 M toy tracks from 1 GeV 18.0 / 18.0.
+constexpr uint32_t k_tail_wide = 8192u;
+inline uint32_t default_tail_tracks(uint64_t n) {
+    return n / 64u < k_tail_wide ? static_cast<uint32_t>(n / 64u)
+                                 : k_tail_wide;
+}
+
 // Whether a plain propagation that asks for direction order is faster without
 // it: where every track tests the same few surfaces an order gains little and
 // scatters the results, unless they are staged or the batch is large.  Input

@@ -484,12 +484,11 @@ __global__ void __launch_bounds__(k_phase_block, sizeof(S) == 4 ? 8 : 4)
 }
 
 // Tail: the tracks left in queue 0, every segment inline.  Up to k_tail_wide
-// tracks a warp runs each (the group form of core/group.cuh): what is left at
-// the end are the longest tracks, and the time is their serial latency.  More
-// than that, one thread per track.  Both kernels are launched and one of them
+// tracks (core/launch_rules.hpp; by default no more are left) a warp runs each
+// (the group form of core/group.cuh): what is left at the end are the longest
+// tracks, and the time is their serial latency.  More than that - a larger
+// tail_tracks, or the last round reached before - one thread per track.  Both kernels are launched and one of them
 // leaves at once, since only the device knows the count.
-constexpr uint32_t k_tail_wide = 8192u;
-
 template <typename S, typename In, bool W>
 __global__ void __launch_bounds__(k_phase_block, 8)
     rounds_tail_kernel(const __grid_constant__ detector_view<S, W> det,
@@ -758,8 +757,6 @@ namespace dprop::api {
 constexpr uint32_t k_default_steps_per_round = 16u;
 constexpr uint32_t k_default_rounds = 64u;
 constexpr uint32_t k_default_yield_lanes = 8u;
-// default tail threshold: n / 64 live tracks
-constexpr uint64_t k_default_tail_div = 64u;
 
 namespace {
 
@@ -820,8 +817,7 @@ dprop_status enqueue_rounds_s(const dprop_launch* lc, const dprop_detector* det,
     const uint32_t sort_interval = lc ? lc->sort_interval : 0u;
     // live tracks below which a round runs the rest to their end
     const uint32_t tail_tracks =
-        (lc && lc->tail_tracks) ? lc->tail_tracks
-                                : static_cast<uint32_t>(n / k_default_tail_div);
+        (lc && lc->tail_tracks) ? lc->tail_tracks : default_tail_tracks(n);
     if (rounds > 100000u || yield > 32u) {
         return fail(DPROP_E_INVALID,
                     "persistent method: rounds > 100000 or yield_lanes > 32");

@@ -196,7 +196,7 @@ def make_launch(method: int = abi.METHOD_PLAIN, block_size: int = 0,
     (double track tensors and results).  steps_per_round, rounds,
     yield_lanes, sort_interval and tail_tracks shape the persistent
     (round-based) method; 0 picks the library default (sort_interval 0: no
-    re-sort by volume; tail_tracks 0: n / 64)."""
+    re-sort by volume; tail_tracks 0: n / 64, at most 8192)."""
     lc = abi.Launch()
     lc.method = method
     lc.block_size = block_size

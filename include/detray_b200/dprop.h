@@ -375,7 +375,8 @@ typedef struct dprop_launch {
     uint32_t tail_tracks;        /* once fewer tracks than this are alive at
                                     the start of a round, they are left to the
                                     kernels after the last round, which run
-                                    them to their end (0: n_tracks / 64;
+                                    them to their end (0: n_tracks / 64, at
+                                    most 8192;
                                     1: only after `rounds` rounds)            */
     uint32_t reserved[1];
 } dprop_launch;

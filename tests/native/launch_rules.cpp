@@ -12,6 +12,8 @@ extern "C" int plain_budget_of(const dprop_detector_desc* d, int extra_code,
                         tracks_per_sm);
 }
 
+extern "C" uint32_t tail_of(uint64_t n) { return default_tail_tracks(n); }
+
 extern "C" int drops_order(const dprop_detector_desc* d, int staged,
                            uint64_t n) {
     return order_is_a_loss(launch_traits_of(d, false), staged != 0, n) ? 1 : 0;

@@ -42,6 +42,7 @@ def rules(tmp_path_factory):
         return bool(lib.drops_order(C.byref(desc.desc), staged,
                                     C.c_uint64(n)))
 
+    get.tail = lambda n: lib.tail_of(C.c_uint64(n))
     get.budget = budget
     get.drops_order = drops_order
     get.load = geometry.load_geometry
@@ -146,3 +147,12 @@ def test_requested_order_is_kept(rules):
     lists = _grids_as_lists(toy, rules.abi)
     for n in (3000, 14000, 300000):
         assert not rules.drops_order(lists, 0, n)
+
+
+def test_default_tail_fits_the_warp_per_track_kernel(rules):
+    """What is left after the last round by default is no more than the kernel
+    with a warp per track takes (8192 tracks), at any batch size."""
+    assert rules.tail(0) == 0 and rules.tail(64) == 1
+    assert rules.tail(200000) == 3125 and rules.tail(524287) == 8191
+    for n in (524288, 524352, 1000000, 2000000, 2**31 - 1):
+        assert rules.tail(n) == 8192
