@@ -525,7 +525,8 @@ def launch_fields(lc):
             "steps_per_round": int(lc.steps_per_round),
             "yield_lanes": int(lc.yield_lanes),
             "rounds": int(lc.rounds),
-            "sort_interval": int(lc.sort_interval)}
+            "sort_interval": int(lc.sort_interval),
+            "by_size": int(lc.by_size)}
 
 
 def config3_row(args, dev, stream, world):

@@ -273,7 +273,7 @@ class Launch(C.Structure):
         ("yield_lanes", C.c_uint32),
         ("sort_interval", C.c_uint32),
         ("tail_tracks", C.c_uint32),
-        ("reserved", C.c_uint32 * 1),
+        ("by_size", C.c_uint32),
     ]
 
 

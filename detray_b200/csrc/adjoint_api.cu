@@ -163,7 +163,7 @@ void launch_adjoint_mb(unsigned int grid, cudaStream_t st,
 extern "C" {
 
 dprop_status dprop_propagate_adjoint(const dprop_config* cfg,
-                                     const dprop_launch* lc,
+                                     const dprop_launch* launch,
                                      const dprop_detector* det,
                                      const dprop_field* field,
                                      const dprop_tracks* tracks,
@@ -210,6 +210,8 @@ dprop_status dprop_propagate_adjoint(const dprop_config* cfg,
     if (n > 0x7fffffffull * k_adj_block) {
         return fail(DPROP_E_INVALID, "propagate_adjoint: too many tracks");
     }
+    const api::launch_request request(launch);
+    const dprop_launch* lc = request.get();
     const cudaStream_t st = static_cast<cudaStream_t>(stream);
     const api::io_ptrs<float> io = api::make_io<float>(*tracks, *results);
     tape_view<float> tv;

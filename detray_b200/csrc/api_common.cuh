@@ -20,6 +20,16 @@ namespace dprop::api {
 dprop_status fail(dprop_status s, const std::string& msg);
 dprop_status cuda_fail(cudaError_t e, const char* what);
 
+// The launch, with its shape left open if by_size says so.
+struct launch_request {
+    explicit launch_request(const dprop_launch* lc);
+    const dprop_launch* get() const { return given_ ? &shape_ : nullptr; }
+
+private:
+    dprop_launch shape_{};
+    bool given_;
+};
+
 // Register budget of a launch: resident CTAs of 128 threads per SM, one of
 // 8 (64 registers), 12 (40) or 16 (32).
 int occupancy_of(const dprop_launch* lc);

@@ -1551,7 +1551,8 @@ dprop_status dprop_autotune(const dprop_config* cfg, const dprop_detector* det,
     // plain: register budget (resident CTAs per SM) x block size x
     // direction sort; persistent: step-phase register budget x steps per
     // round x tracks per warp (yield lanes) x rounds x volume re-sort
-    // interval x direction sort
+    // interval x direction sort; candidate k_by_size leaves the shape open
+    constexpr int k_by_size = 1;
     struct cand {
         uint32_t method, block, ctas, sort, steps, yield, rounds, interval;
     };
@@ -1585,11 +1586,14 @@ dprop_status dprop_autotune(const dprop_config* cfg, const dprop_detector* det,
         lc.steps_per_round = cands[i].steps;
         lc.yield_lanes = cands[i].yield;
         lc.rounds = cands[i].rounds;
-        s = launch<float>(*cfg, &lc, det, field, io, m, stream);  // warm-up
+        lc.by_size = i == k_by_size ? 1u : 0u;
+        const dprop::api::launch_request request(&lc);
+        const dprop_launch* shape = request.get();
+        s = launch<float>(*cfg, shape, det, field, io, m, stream);  // warm-up
         if (s != DPROP_OK) break;
         cudaEventRecord(e0, stream);
         for (int k = 0; k < 2 && s == DPROP_OK; ++k) {
-            s = launch<float>(*cfg, &lc, det, field, io, m, stream);
+            s = launch<float>(*cfg, shape, det, field, io, m, stream);
         }
         cudaEventRecord(e1, stream);
         const cudaError_t ce = cudaEventSynchronize(e1);
@@ -1620,6 +1624,7 @@ dprop_status dprop_autotune(const dprop_config* cfg, const dprop_detector* det,
     launch_out->steps_per_round = cands[best_i].steps;
     launch_out->yield_lanes = cands[best_i].yield;
     launch_out->rounds = cands[best_i].rounds;
+    launch_out->by_size = best_i == k_by_size ? 1u : 0u;
     return DPROP_OK;
 }
 
@@ -1719,11 +1724,14 @@ dprop_status dprop_field_destroy(dprop_field* f) {
     return DPROP_OK;
 }
 
-dprop_status dprop_propagate(const dprop_config* cfg, const dprop_launch* lc,
+dprop_status dprop_propagate(const dprop_config* cfg,
+                             const dprop_launch* launch_cfg,
                              const dprop_detector* det, const dprop_field* field,
                              const dprop_tracks* tracks,
                              const dprop_results* results, uint64_t n,
                              void* stream) {
+    const dprop::api::launch_request request(launch_cfg);
+    const dprop_launch* lc = request.get();
     dprop_status s = check_config(cfg);
     if (s != DPROP_OK) {
         return s;
@@ -1756,11 +1764,13 @@ dprop_status dprop_propagate(const dprop_config* cfg, const dprop_launch* lc,
 }
 
 dprop_status dprop_propagate_host(const dprop_config* cfg,
-                                  const dprop_launch* lc,
+                                  const dprop_launch* launch_cfg,
                                   const dprop_detector* det,
                                   const dprop_field* field,
                                   const dprop_tracks* tracks,
                                   const dprop_results* results, uint64_t n) {
+    const dprop::api::launch_request request(launch_cfg);
+    const dprop_launch* lc = request.get();
     dprop_status s = check_config(cfg);
     if (s != DPROP_OK) {
         return s;

@@ -49,6 +49,18 @@ void launch_group(cudaStream_t st, const dprop_detector* det,
 
 namespace dprop::api {
 
+launch_request::launch_request(const dprop_launch* lc) : given_(lc != nullptr) {
+    if (!lc) {
+        return;
+    }
+    shape_ = *lc;
+    if (shape_.by_size == 1u) {
+        shape_.block_size = shape_.ctas_per_sm = shape_.steps_per_round = 0u;
+        shape_.rounds = shape_.yield_lanes = shape_.sort_interval = 0u;
+        shape_.tail_tracks = shape_.by_size = 0u;
+    }
+}
+
 bool open_shape(const dprop_launch* lc) {
     return !lc || (lc->block_size | lc->ctas_per_sm | lc->steps_per_round |
                    lc->rounds | lc->yield_lanes | lc->sort_interval |

@@ -537,7 +537,8 @@ def propagate_host(cfg: abi.Config, det: Detector, field: Field,
 
 # the candidates dprop_autotune times, in its order: (method, block_size,
 # ctas_per_sm, sort_tracks, steps_per_round, yield_lanes, rounds,
-# sort_interval)
+# sort_interval); the second one runs with by_size set, the form that follows
+# the batch size
 AUTOTUNE_CANDIDATES = [
     ("plain", 128, 8, 1, 0, 0, 0, 0), ("plain", 128, 12, 1, 0, 0, 0, 0),
     ("plain", 128, 16, 1, 0, 0, 0, 0), ("plain", 256, 16, 1, 0, 0, 0, 0),

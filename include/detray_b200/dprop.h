@@ -378,7 +378,11 @@ typedef struct dprop_launch {
                                     them to their end (0: n_tracks / 64, at
                                     most 8192;
                                     1: only after `rounds` rounds)            */
-    uint32_t reserved[1];
+    uint32_t by_size;            /* 1: as if block_size, ctas_per_sm and the
+                                    persistent fields above were 0, whatever
+                                    they hold: the form follows the batch size
+                                    (dprop_autotune sets it where that was the
+                                    fastest)                                   */
 } dprop_launch;
 
 /* ------------------------------------------------------------------ API */
@@ -586,15 +590,17 @@ dprop_status dprop_propagate_noalloc(const dprop_config* cfg,
 
 /* Autotuner: times candidate launch forms - the plain kernel at the three
  * register budgets (ctas_per_sm 8, 12, 16) with the direction sort, at 16
- * with 256-thread blocks and at 16 without the sort; the persistent method
+ * with 256-thread blocks and at 16 without the sort, the one at 12 with
+ * by_size set (the form that follows the batch size: small batches run a warp
+ * per track, which no spelled-out shape is); the persistent method
  * with and without the sort over its step-phase register budget
  * (ctas_per_sm 3, 4, 5), steps per round, tracks per warp (yield_lanes 8,
  * 12, 16), the volume re-sort interval (0, 1, 2) and the number of rounds
  * before the tail kernel - on the first min(n_tracks, 1048576) of the given
  * device tracks (under a CUDA graph if launch->use_graph is set), and writes
  * the fastest into *launch (method, block_size, ctas_per_sm, sort_tracks,
- * steps_per_round, yield_lanes, rounds, sort_interval; use_graph is left as
- * given).  If timings_ms is not NULL it receives one time per candidate
+ * steps_per_round, yield_lanes, rounds, sort_interval, by_size; use_graph is
+ * left as given).  If timings_ms is not NULL it receives one time per candidate
  * (DPROP_AUTOTUNE_CANDIDATES entries).  Allocates temporary device result
  * buffers for the trial runs. */
 #define DPROP_AUTOTUNE_CANDIDATES 13
