@@ -183,4 +183,15 @@ inline int plain_budget(const launch_traits& t, bool field_map,
     return field_map && t.surface_grids && tracks_per_sm >= 1536u ? 16 : 8;
 }
 
+// Device scratch of a host call without jagged records: inputs (8 doubles a
+// track), per-track outputs (status, six counters, path length, the 8 final
+// parameters) and records (barcode, 6 + 21 + 1 floats, flags), each array
+// from a 256-byte boundary on.
+inline uint64_t host_scratch_bytes(uint64_t n, uint64_t max_records) {
+    const auto al = [](uint64_t b) { return (b + 255u) & ~uint64_t(255u); };
+    const uint64_t r = max_records * n;
+    return 8u * al(8u * n) + al(n) + 15u * al(4u * n) + al(8u * r) +
+           28u * al(4u * r) + al(r);
+}
+
 }  // namespace dprop

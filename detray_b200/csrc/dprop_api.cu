@@ -1788,11 +1788,7 @@ dprop_status dprop_propagate_host(const dprop_config* cfg,
         return propagate_host_jagged(*cfg, lc, det, field, *tracks, *results, n);
     }
     const uint64_t cap = cfg->max_records;
-    // device scratch: inputs (8 doubles), per-track outputs, records
-    const size_t in_bytes = 8 * n * sizeof(double);
-    const size_t trk_bytes = n * (1 + 6 * 4 + 4 + 8 * 4) + 16 * 256;
-    const size_t rec_bytes = cap * n * (8 + 6 * 4 + 21 * 4 + 4 + 1);
-    s = ensure_scratch(in_bytes + trk_bytes + rec_bytes + 4096);
+    s = ensure_scratch(host_scratch_bytes(n, cap));
     if (s != DPROP_OK) {
         return s;
     }

@@ -14,6 +14,10 @@ extern "C" int plain_budget_of(const dprop_detector_desc* d, int extra_code,
 
 extern "C" uint32_t tail_of(uint64_t n) { return default_tail_tracks(n); }
 
+extern "C" uint64_t host_scratch(uint64_t n, uint64_t max_records) {
+    return host_scratch_bytes(n, max_records);
+}
+
 extern "C" int drops_order(const dprop_detector_desc* d, int staged,
                            uint64_t n) {
     return order_is_a_loss(launch_traits_of(d, false), staged != 0, n) ? 1 : 0;

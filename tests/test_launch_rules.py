@@ -43,6 +43,9 @@ def rules(tmp_path_factory):
                                     C.c_uint64(n)))
 
     get.tail = lambda n: lib.tail_of(C.c_uint64(n))
+    lib.host_scratch.restype = C.c_uint64
+    get.host_scratch = lambda n, r: lib.host_scratch(C.c_uint64(n),
+                                                     C.c_uint64(r))
     get.budget = budget
     get.drops_order = drops_order
     get.load = geometry.load_geometry
@@ -156,3 +159,16 @@ def test_default_tail_fits_the_warp_per_track_kernel(rules):
     assert rules.tail(200000) == 3125 and rules.tail(524287) == 8191
     for n in (524288, 524352, 1000000, 2000000, 2**31 - 1):
         assert rules.tail(n) == 8192
+
+
+@pytest.mark.parametrize("n", [1, 3, 63, 64, 65, 1000, 4097])
+@pytest.mark.parametrize("max_records", [0, 1, 7, 16, 32])
+def test_host_scratch_holds_every_array(rules, n, max_records):
+    """The arrays of a host call, each from a 256-byte boundary on."""
+    r = n * max_records
+    sizes = ([8 * n] * 8 + [n] + [4 * n] * (6 + 1 + 8)
+             + [8 * r] + [4 * r] * (6 + 21 + 1) + [r])
+    end = 0
+    for s in sizes:
+        end += -(-s // 256) * 256
+    assert rules.host_scratch(n, max_records) >= end
