@@ -672,12 +672,12 @@ struct surface_walk {
     }
     template <bool W>
     DPROP_HD uint32_t next(const detector_view<S, W>& det,
-                           const dev_grid<S>& g) {
+                           const dev_grid<S>* g) {
         while (e >= end) {
             if (c >= n_bins) {
                 return k_invalid;
             }
-            const uint32_t b = window_bin(g, i0, i1);
+            const uint32_t b = window_bin(*g, i0, i1);
             ++c;
             if (++i1 == hi1) {
                 i1 = lo1;
@@ -685,7 +685,7 @@ struct surface_walk {
             }
             const uint32_t v = det.grid_bins[b];
             if constexpr (W) {
-                if (g.multi) {
+                if (g->multi) {
                     list = det.grid_bins;
                     e = v;
                     end = det.grid_bins[b + 1u];
@@ -713,10 +713,10 @@ DPROP_HD_COLD void local_navigation(nav_state<S>& nav, const detector_view<S, W>
     const vec3<S> ro = trk.pos;
     const vec3<S> rd = nav.direction * trk.dir;
     const bool has_grid = vol.grid != k_invalid;
-    const dev_grid<S>& grid = det.grids[has_grid ? vol.grid : 0u];
-    bin_window w{0, 0, 0, 0};
+    const dev_grid<S>* const grid = has_grid ? det.grids + vol.grid : nullptr;
+    bin_window w{0, 0, 0, 0};  // no bins without a grid
     if (has_grid) {
-        w = grid_window(det, grid, trk, cfg);
+        w = grid_window(det, *grid, trk, cfg);
     }
     if constexpr (G::lanes == 1) {
         surface_walk<S> walk;
@@ -732,7 +732,7 @@ DPROP_HD_COLD void local_navigation(nav_state<S>& nav, const detector_view<S, W>
         const int n_bins = (w.hi0 - w.lo0) * span;
         auto bin_of = [&](int c) {
             const int row = c / span;
-            return window_bin(grid, w.lo0 + row, w.lo1 + (c - row * span));
+            return window_bin(*grid, w.lo0 + row, w.lo1 + (c - row * span));
         };
         if constexpr (W) {
             // lists: 0 the brute-force list, 1 + c the bins; a list per
@@ -746,8 +746,8 @@ DPROP_HD_COLD void local_navigation(nav_state<S>& nav, const detector_view<S, W>
                 } else if (l <= n_bins) {
                     const uint32_t b = bin_of(l - 1);
                     const uint32_t v = det.grid_bins[b];
-                    e0 = grid.multi ? v : b;
-                    e1 = grid.multi ? det.grid_bins[b + 1u]
+                    e0 = grid->multi ? v : b;
+                    e1 = grid->multi ? det.grid_bins[b + 1u]
                                     : (v != k_invalid ? b + 1u : b);
                 }
                 // entry f of the pass: in the lane whose scanned counts
