@@ -554,14 +554,15 @@ DPROP_HD int axis_bin(S v, S lo, S hi, uint32_t n) {
     const S width = (hi - lo) / static_cast<S>(n);
     const S u = (v - lo) / width + S(1);
     // out-of-range values (a failed reference-surface intersection) are
-    // saturated instead of overflowing the integer conversion
+    // saturated instead of overflowing the integer conversion, far enough
+    // from its limits for a search window either side of them
     int b;
     if (!(u == u)) {
         b = 0;
-    } else if (u >= S(2147483000)) {
-        b = 2147483000;
-    } else if (u <= S(-2147483000)) {
-        b = -2147483000;
+    } else if (u >= S(1073741824)) {
+        b = 1073741824;
+    } else if (u <= S(-1073741824)) {
+        b = -1073741824;
     } else {
         b = static_cast<int>(u);
     }

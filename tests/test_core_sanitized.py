@@ -36,10 +36,21 @@ child({lib!r}, {case!r}, {precision})
 
 def _case(case):
     from detray_b200 import abi, geometry, tracks
-    # a detector without any grid
-    return (geometry.load_geometry("telescope_10x1m_300um"),
-            tracks.telescope_tracks(50, seed=1),
-            abi.make_config(max_records=16))
+    if case == "telescope":  # a detector without any grid
+        return (geometry.load_geometry("telescope_10x1m_300um"),
+                tracks.telescope_tracks(50, seed=1),
+                abi.make_config(max_records=16))
+    # tracks along the discs of an endcap: the grid's reference plane is not
+    # reached, and the wide window starts from a bin far outside
+    trk = tracks.toy_tracks(20, seed=2)
+    trk[0:2] = 0.0
+    trk[0] = 60.0
+    trk[2] = np.linspace(610.0, 1400.0, 20)
+    trk[4:7] = 0.0
+    trk[4] = 1.0
+    trk[7] = 1e-4
+    return (geometry.load_geometry("toy_4brl_7edc"), trk,
+            abi.make_config(max_records=16, search_window=(700, 700)))
 
 
 def child(path, case, precision):
@@ -60,7 +71,7 @@ def child(path, case, precision):
     sys.exit(0 if rc == 0 else 3)
 
 
-@pytest.mark.parametrize("case", ["telescope"])
+@pytest.mark.parametrize("case", ["telescope", "along_discs"])
 @pytest.mark.parametrize("precision", [4, 8])
 def test_no_undefined_behaviour(lib, case, precision):
     p = subprocess.run([sys.executable, "-c",
