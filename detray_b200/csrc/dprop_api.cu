@@ -1921,6 +1921,31 @@ static_assert(k_noalloc_temp_offset < DPROP_NOALLOC_SCRATCH_BYTES,
 static __device__ __align__(256) unsigned char
     g_noalloc_scratch[DPROP_NOALLOC_SCRATCH_BYTES];
 
+// Every kernel the entry point may choose by detector, configuration and batch
+// size, run on no track: the driver loads a kernel's code, and reserves the
+// local memory it needs, at its first launch - which would otherwise be an
+// allocation in the middle of a run, at the first batch of another size.
+template <int MB, bool Grad>
+void launch_empty_plain(cudaStream_t st) {
+    const field_view<float> field{};
+    const prop_cfg<float> cfg{};
+    const io_ptrs<float> io{};
+    const dprop::api::stage_ptrs stage{};
+    propagate_plain_kernel<float, MB, true, Grad><<<1, k_plain_block, 0, st>>>(
+        detector_view<float, true>{}, field, cfg, io, 0u, nullptr, stage);
+    propagate_plain_kernel<float, MB, false, Grad><<<1, k_plain_block, 0, st>>>(
+        detector_view<float, false>{}, field, cfg, io, 0u, nullptr, stage);
+}
+
+dprop_status load_noalloc_forms(cudaStream_t st) {
+    launch_empty_plain<4, false>(st);
+    launch_empty_plain<8, false>(st);
+    launch_empty_plain<16, false>(st);
+    launch_empty_plain<8, true>(st);
+    DPROP_CUDA(cudaGetLastError());
+    return dprop::api::load_group_forms(st);
+}
+
 constexpr int k_noalloc_max_devices = 64;
 void* g_noalloc_device_ptr[k_noalloc_max_devices] = {};
 std::mutex g_noalloc_mutex;
@@ -1946,6 +1971,13 @@ dprop_status noalloc_scratch(cudaStream_t stream, void** out) {
         const cudaError_t e = cudaGetSymbolAddress(&p, g_noalloc_scratch);
         if (e != cudaSuccess) {
             return cuda_fail(e, "cudaGetSymbolAddress(no-alloc scratch)");
+        }
+        if (g_noalloc_device_ptr[dev] != p) {
+            // the first call on the device (or after a reset of it)
+            const dprop_status s = load_noalloc_forms(stream);
+            if (s != DPROP_OK) {
+                return s;
+            }
         }
         g_noalloc_device_ptr[dev] = p;
     } else if (g_noalloc_device_ptr[dev] == nullptr) {

@@ -27,8 +27,10 @@ __global__ void __launch_bounds__(32, MinBlocks)
                            const __grid_constant__ prop_cfg<float> cfg,
                            const __grid_constant__ api::io_ptrs<In> io,
                            uint64_t n) {
-    api::run_group<In>(blockIdx.x, n, det, field, cfg, io,
-                       lane_group<32>::make(threadIdx.x));
+    if (blockIdx.x < n) {
+        api::run_group<In>(blockIdx.x, n, det, field, cfg, io,
+                           lane_group<32>::make(threadIdx.x));
+    }
 }
 
 template <int MinBlocks, typename In>
@@ -45,9 +47,28 @@ void launch_group(cudaStream_t st, const dprop_detector* det,
     }
 }
 
+template <int MinBlocks>
+void launch_empty_group(cudaStream_t st) {
+    const field_view<float> field{};
+    const prop_cfg<float> cfg{};
+    const api::io_ptrs<float> io{};
+    propagate_group_kernel<float, true, MinBlocks><<<1, 32, 0, st>>>(
+        detector_view<float, true>{}, field, cfg, io, 0u);
+    propagate_group_kernel<float, false, MinBlocks><<<1, 32, 0, st>>>(
+        detector_view<float, false>{}, field, cfg, io, 0u);
+}
+
 }  // namespace
 
 namespace dprop::api {
+
+dprop_status load_group_forms(cudaStream_t st) {
+    launch_empty_group<16>(st);
+    launch_empty_group<20>(st);
+    launch_empty_group<32>(st);
+    DPROP_CUDA(cudaGetLastError());
+    return DPROP_OK;
+}
 
 launch_request::launch_request(const dprop_launch* lc) : given_(lc != nullptr) {
     if (!lc) {

@@ -562,7 +562,8 @@ dprop_status dprop_validate_navigation(const dprop_scan_results* truth,
  * cudaMalloc or cudaFree (which can synchronise the whole device) is not
  * acceptable, or an application that fixes its device-memory budget up
  * front.  It does what dprop_propagate does with sort_tracks = 1 and the
- * plain one-thread-per-track kernel, but the scratch the direction sort needs
+ * plain method (a warp per track for small batches, one thread per track
+ * else; results are not staged), but the scratch the direction sort needs
  * (keys, indices, radix-sort temporary storage) lives in one fixed array
  * compiled into the library: DPROP_NOALLOC_SCRATCH_BYTES on every GPU that
  * loads the library, held until the process exits.  Inputs and outputs are
@@ -570,6 +571,9 @@ dprop_status dprop_validate_navigation(const dprop_scan_results* truth,
  *
  *  - At most DPROP_NOALLOC_MAX_TRACKS tracks per call; a larger batch is
  *    rejected with DPROP_E_INVALID (split it into several calls).
+ *  - The first call on a device outside a stream capture loads the code of
+ *    every kernel the entry point may choose for later batches, detectors and
+ *    configurations, and has the driver reserve their local memory.
  *  - Each call outside a stream capture looks up the device's copy of the
  *    array (a call inside a capture reuses the last address found on that
  *    device); make the first call on a device before capturing any stream
