@@ -17,7 +17,6 @@
 //                             atomics per surface
 #include <cuda_runtime.h>
 
-#include <mutex>
 
 #include "api_common.cuh"
 #include "core/config.hpp"
@@ -115,16 +114,8 @@ __global__ void __launch_bounds__(k_adj_block)
     }
 }
 
-// Library-owned, grow-only device scratch of the direction sort in adjoint
-// mode (one per process; calls are serialised by the mutex on the host side
-// and the scratch is only reused after the caller's stream reached it).
-struct adj_sort_scratch {
-    void* buf{nullptr};
-    size_t bytes{0};
-    int device{-1};
-};
-adj_sort_scratch g_adj_sort;
-std::mutex g_adj_mutex;
+// kept between calls: the direction sort's scratch in adjoint mode
+api::kept_scratch g_adj_sort{api::staging_area()};
 
 // MB: resident CTAs per SM; with the field gradient 2 (255 registers), 4 or 8.
 template <int MB>
@@ -240,27 +231,17 @@ dprop_status dprop_propagate_adjoint(const dprop_config* cfg,
         return DPROP_OK;
     }
 
-    std::lock_guard<std::mutex> lock(g_adj_mutex);
+    api::kept_scratch::use sort_use;
     const uint32_t* order = nullptr;
     if (lc && lc->sort_tracks) {
         const size_t need = api::sort_scratch_bytes(n);
-        if (g_adj_sort.bytes < need || g_adj_sort.device != dev) {
-            if (g_adj_sort.buf) {
-                DPROP_CUDA(cudaStreamSynchronize(st));
-                cudaFree(g_adj_sort.buf);
-                g_adj_sort.buf = nullptr;
-                g_adj_sort.bytes = 0;
-            }
-            DPROP_CUDA(api::alloc_device(&g_adj_sort.buf, need));
-            g_adj_sort.bytes = need;
-            g_adj_sort.device = dev;
-        }
+        DPROP_CUDA(g_adj_sort.take(need, st, &sort_use));
         const dprop_status s = api::enqueue_direction_sort(
             static_cast<const float*>(tracks->dir[0]),
             static_cast<const float*>(tracks->dir[1]),
             static_cast<const float*>(tracks->dir[2]),
-            static_cast<const float*>(tracks->qop), n, g_adj_sort.buf,
-            g_adj_sort.bytes, st, &order);
+            static_cast<const float*>(tracks->qop), n, sort_use.buf, need, st,
+            &order);
         if (s != DPROP_OK) {
             return s;
         }

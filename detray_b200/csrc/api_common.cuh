@@ -83,6 +83,9 @@ private:
     std::vector<void*> retired_;   // outgrown, but in a captured graph
 };
 
+// The staging area of sorted plain propagations.
+kept_scratch* staging_area();
+
 // cudaMalloc; without room for it the staging area of sorted propagations, an
 // option that is kept between calls, is given back first.
 cudaError_t alloc_device(void** p, size_t bytes);

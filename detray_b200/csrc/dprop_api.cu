@@ -201,20 +201,25 @@ dprop_status ensure_scratch(size_t bytes) {
     return DPROP_OK;
 }
 
-// Kept between calls: the staged results of sorted plain propagations, the
-// direction sort's scratch, the slots and queues of the persistent method.  A
-// call that needs two takes the sort's first, the staging area last.
-dprop::api::kept_scratch g_stage;
-dprop::api::kept_scratch g_sort{&g_stage};
-dprop::api::kept_scratch g_rounds{&g_stage};
+// Kept between calls: the direction sort's scratch, the slots and queues of the
+// persistent method and (staging_area) the staged results of sorted plain
+// propagations.  A call that needs two takes the sort's first, the staging
+// area last.
+dprop::api::kept_scratch g_sort{dprop::api::staging_area()};
+dprop::api::kept_scratch g_rounds{dprop::api::staging_area()};
 
 }  // namespace
 
 namespace dprop::api {
 
+kept_scratch* staging_area() {
+    static kept_scratch area;
+    return &area;
+}
+
 cudaError_t alloc_device(void** p, size_t bytes) {
     cudaError_t e = cudaMalloc(p, bytes);
-    if (e == cudaErrorMemoryAllocation && g_stage.give_back()) {
+    if (e == cudaErrorMemoryAllocation && staging_area()->give_back()) {
         cudaGetLastError();
         e = cudaMalloc(p, bytes);
     }
@@ -734,8 +739,10 @@ dprop_status launch(const dprop_config& c, const dprop_launch* launch_cfg,
         }
         scr.rounds_bytes = work_bytes();
         if (scr.rounds_bytes > 0) {
-            const cudaError_t e = (plan.rounds ? g_rounds : g_stage)
-                                      .take(scr.rounds_bytes, stream, &work_use);
+            dprop::api::kept_scratch* work =
+                plan.rounds ? &g_rounds : dprop::api::staging_area();
+            const cudaError_t e =
+                work->take(scr.rounds_bytes, stream, &work_use);
             if (e == cudaErrorMemoryAllocation && !plan.rounds) {
                 // staging is an option: without room for it the results go
                 // to the caller's arrays directly
@@ -1885,7 +1892,7 @@ dprop_status dprop_release_cache(void) {
     g_graphs.clear();
     g_sort.release();
     g_rounds.release();
-    g_stage.release();
+    dprop::api::staging_area()->release();
     cudaFree(g_scratch.buf);
     g_scratch.buf = nullptr;
     g_scratch.bytes = 0;

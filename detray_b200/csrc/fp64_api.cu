@@ -13,7 +13,6 @@
 //                              (dprop_launch.method = DPROP_METHOD_PERSISTENT)
 #include <cuda_runtime.h>
 
-#include <mutex>
 #include <type_traits>
 
 #include "api_common.cuh"
@@ -56,33 +55,10 @@ __global__ void __launch_bounds__(32, MinBlocks)
                            lane_group<32>::make(threadIdx.x));
 }
 
-// library-owned grow-only sort scratch of fp64 launches
-struct f64_sort_scratch {
-    void* buf{nullptr};
-    size_t bytes{0};
-    int device{-1};
-};
-f64_sort_scratch g_f64_sort;
-f64_sort_scratch g_f64_rounds;  // persistent method: slots and queues
-std::mutex g_f64_mutex;
-
-dprop_status ensure_f64(f64_sort_scratch& sc, size_t need,
-                        cudaStream_t stream) {
-    int dev = 0;
-    DPROP_CUDA(cudaGetDevice(&dev));
-    if (sc.bytes < need || sc.device != dev) {
-        if (sc.buf) {
-            DPROP_CUDA(cudaStreamSynchronize(stream));
-            cudaFree(sc.buf);
-            sc.buf = nullptr;
-            sc.bytes = 0;
-        }
-        DPROP_CUDA(api::alloc_device(&sc.buf, need));
-        sc.bytes = need;
-        sc.device = dev;
-    }
-    return DPROP_OK;
-}
+// kept between fp64 calls: the direction sort's scratch, and the persistent
+// method's slots and queues; a call takes the sort's first
+api::kept_scratch g_f64_sort{api::staging_area()};
+api::kept_scratch g_f64_rounds{api::staging_area()};
 
 }  // namespace
 
@@ -124,17 +100,14 @@ dprop_status propagate_fp64(const dprop_config& c, const dprop_launch* lc,
         DPROP_CUDA(cudaGetLastError());
         return DPROP_OK;
     }
-    std::lock_guard<std::mutex> lock(g_f64_mutex);
+    kept_scratch::use sort_use, rounds_use;
     const uint32_t* order = nullptr;
     if (lc && lc->sort_tracks) {
-        const dprop_status e =
-            ensure_f64(g_f64_sort, sort_scratch_bytes(n), stream);
-        if (e != DPROP_OK) {
-            return e;
-        }
+        const size_t need = sort_scratch_bytes(n);
+        DPROP_CUDA(g_f64_sort.take(need, stream, &sort_use));
         const dprop_status s = enqueue_direction_sort(
-            io.trk[4], io.trk[5], io.trk[6], io.trk[7], n, g_f64_sort.buf,
-            g_f64_sort.bytes, stream, &order);
+            io.trk[4], io.trk[5], io.trk[6], io.trk[7], n, sort_use.buf, need,
+            stream, &order);
         if (s != DPROP_OK) {
             return s;
         }
@@ -143,13 +116,9 @@ dprop_status propagate_fp64(const dprop_config& c, const dprop_launch* lc,
         !(open && n < rounds_from_fp64(det->traits))) {
         const size_t need = rounds_scratch_bytes_fp64(
             n, det->wires, staged_capacity(pc, io));
-        const dprop_status e = ensure_f64(g_f64_rounds, need, stream);
-        if (e != DPROP_OK) {
-            return e;
-        }
+        DPROP_CUDA(g_f64_rounds.take(need, stream, &rounds_use));
         return enqueue_rounds_fp64(lc, det, field, pc, io, n, order,
-                                   g_f64_rounds.buf, g_f64_rounds.bytes,
-                                   stream);
+                                   rounds_use.buf, need, stream);
     }
     const unsigned int grid =
         static_cast<unsigned int>((n + k_f64_block - 1) / k_f64_block);
@@ -191,11 +160,8 @@ dprop_status propagate_fp64(const dprop_config& c, const dprop_launch* lc,
 }
 
 void release_fp64_scratch() {
-    std::lock_guard<std::mutex> lock(g_f64_mutex);
-    for (f64_sort_scratch* sc : {&g_f64_sort, &g_f64_rounds}) {
-        cudaFree(sc->buf);
-        *sc = f64_sort_scratch{};
-    }
+    g_f64_sort.release();
+    g_f64_rounds.release();
 }
 
 }  // namespace dprop::api

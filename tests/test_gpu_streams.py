@@ -125,3 +125,48 @@ def test_captured_sorted_call(setup):
     for k, x in want.tensors.items():
         assert torch.equal(x.view(torch.uint8),
                            res.tensors[k].view(torch.uint8)), k
+
+
+@pytest.mark.parametrize("form", ["fp64_plain", "fp64_rounds", "adjoint"])
+def test_overlapping_calls_of_the_other_kernels(setup, form):
+    """Double precision and the adjoint keep their own sort scratch and
+    slots: two streams, sorted calls in turn."""
+    torch = setup[0]
+    from detray_b200 import abi, adjoint, geometry, propagator, tracks
+    from detray_b200.units import T
+    det = propagator.Detector(geometry.load_geometry("toy_4brl_7edc"))
+    field = propagator.Field.constant((0.0, 0.0, 2.0 * T))
+    cfg = abi.make_config(max_records=16, search_window=(3, 3),
+                          estimate_scattering_noise=0)
+    dtype = torch.float32 if form == "adjoint" else torch.float64
+    shape = dict(method=1, ctas_per_sm=2) if form == "fp64_rounds" else {}
+    launch = propagator.make_launch(
+        sort_tracks=1, precision=8 if dtype == torch.float64 else 0, **shape)
+    trk = [torch.tensor(tracks.toy_tracks(20000, seed=s), dtype=dtype,
+                        device="cuda") for s in (35, 36)]
+
+    def call(side, stream):
+        with torch.cuda.stream(stream):
+            if form == "adjoint":
+                return adjoint.propagate_adjoint(cfg, det, field, trk[side],
+                                                 launch).results.tensors
+            return propagator.propagate(cfg, det, field, trk[side],
+                                        launch=launch).tensors
+
+    streams = [torch.cuda.Stream() for _ in trk]
+    torch.cuda.synchronize()
+    alone = []
+    for side in (0, 1):
+        alone.append(call(side, streams[side]))
+        torch.cuda.synchronize()
+    got = [(side, call(side, streams[side])) for _ in range(4)
+           for side in (0, 1)]
+    torch.cuda.synchronize()
+    for side, b in got:
+        a = alone[side]
+        for k in ("status", "n_records", "n_steps", "n_trials",
+                  "n_intersections"):
+            assert torch.equal(a[k], b[k]), k
+        for k in ("path_length", "final_free"):
+            assert torch.equal(a[k].view(torch.uint8),
+                               b[k].view(torch.uint8)), k
