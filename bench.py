@@ -684,9 +684,12 @@ def run_ours(args):
                    "step phase and navigation phase, then the queue builder, "
                    "the tail (2) and the record conversion")
     else:
-        per_step = 1 + 2 * int(lc.sort_tracks)
+        # sorted batches of 16 384 tracks and more stage their results
+        staged = bool(lc.sort_tracks) and n >= 16384
+        per_step = 1 + int(lc.sort_tracks) + int(staged)
         kernels = ("direction key, propagate_plain_kernel, the record "
-                   "conversion (sorted)")
+                   "conversion" if staged else
+                   "direction key, propagate_plain_kernel")
     roofline = {"bound": "fp32", "achieved": round(achieved, 4),
                 "peak": round(peak, 2), "unit": "TFLOP/s",
                 "frac": round(achieved / peak, 5), "traffic": traffic,

@@ -30,8 +30,8 @@ private:
     bool given_;
 };
 
-// Register budget of a launch: resident CTAs of 128 threads per SM, one of
-// 8 (64 registers), 12 (40) or 16 (32).
+// Register budget a launch spells out: resident CTAs of 128 threads per SM, one
+// of 8 (64 registers), 12 (40) or 16 (32).
 int occupancy_of(const dprop_launch* lc);
 
 // Device memory the library keeps between calls: one grow-only buffer per
@@ -197,7 +197,8 @@ struct dprop_field {
 namespace dprop::api {
 
 // fp64 propagation (dprop_launch.precision == 8): double inputs, arithmetic
-// and results; plain one-thread-per-track kernel, optional direction sort.
+// and results; the forms of group_limit_fp64 and rounds_from_fp64
+// (core/launch_rules.hpp), optional direction sort.
 dprop_status propagate_fp64(const dprop_config& cfg, const dprop_launch* lc,
                             const dprop_detector* det, const dprop_field* field,
                             const dprop_tracks& tracks,

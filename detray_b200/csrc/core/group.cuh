@@ -14,11 +14,12 @@
 
 namespace dprop {
 
-// L lanes of a warp, aligned to L: 8, 16 or 32.  All lanes of a group call
-// every member together.
+// The L lanes of a warp that run one track.  All lanes of a group call every
+// member together.  The kernels use whole warps: 8 and 16 lanes per track were
+// never clearly faster at any batch size.
 template <int L>
 struct lane_group {
-    static_assert(L == 8 || L == 16 || L == 32, "group of 8, 16 or 32 lanes");
+    static_assert(L == 32, "a warp per track");
     static constexpr int lanes = L;
     static constexpr bool packed = false;
     uint32_t mask;   // the group's lanes in the warp

@@ -493,9 +493,12 @@ struct scan_probe {
         K_inv = 1.f / K;
         alpha = norm(n);
         delta = dot(h, t);
-        // sine and cosine are good to 1e-6 here, 1/K converts them to mm; a
-        // helix of no curvature, or one that moves along the field axis
-        // (helix::straight), is not tested at all
+        // sine and cosine are good to 1e-6 here, 1/K converts them to mm; for
+        // a helix of no curvature, or one that moves along the field axis
+        // (helix::straight), every sphere is near.  The test of a plane along
+        // the field holds for it as well: a track along the axis keeps its
+        // distance to the plane, and without curvature the terms are not
+        // numbers.
         slack = hx.straight ? limits<float>::max()
                             : 1.f + 4e-6f * fabs(K_inv);
     }

@@ -3,7 +3,10 @@
 // groups they write; the kernels (rounds.cuh) wrap these bodies with the
 // work queues and warp-level scheduling, and the tests run the same bodies
 // on the host in rounds to check that a track driven through them ends
-// bit-identical to propagate_track.
+// bit-identical to propagate_track.  The step phase's bodies take the
+// navigation state in two forms: nav_window (slots.cuh), three candidates
+// held, which the kernels run, and nav_state, the candidate cache as an array
+// of which a window is kept loaded, which only host simulations run.
 //
 //   phase_init   propagation start: track state, navigator initialisation
 //   fast phase   the loop's light segments, RK steps (with the high-trust
@@ -84,8 +87,8 @@ DPROP_HD void phase_init(const slot_soa<S>& s, uint64_t slot, uint32_t track,
 }
 
 // ------------------------------------------------------------------ fast
-// The cached candidates a fast-phase track has in registers: the contiguous
-// cache indices [lo, hi].  A segment reads at most the current surface, the
+// With the candidate cache as an array: the entries a fast-phase track has
+// loaded, the contiguous cache indices [lo, hi].  A segment reads at most the current surface, the
 // target and the candidate after it (reached and re-intersected in the same
 // update), so before each segment the window is grown to cover
 // [next - 1, next + 1]; only the entries it covers are loaded and written
@@ -110,7 +113,7 @@ DPROP_HD void ensure_cands(const slot_soa<S>& s, uint64_t slot,
     w.hi = b > w.hi ? b : w.hi;
 }
 
-// With the candidates in registers the window is nav_window's own.
+// nav_window holds its candidates itself; the window stays unused.
 template <typename S>
 DPROP_HD void ensure_cands(const slot_soa<S>&, uint64_t, nav_window<S>&,
                            cand_window&) {}

@@ -8,7 +8,8 @@
 //                                (tests/benchmarks/include/detray/benchmarks/
 //                                device/cuda/propagation_benchmark.cu:13-68)
 // The persistent method's round-based phase kernels are in rounds.cuh, the
-// warp-per-track form of small batches in group_api.cu.  All write the slot-major records of dprop_results.
+// warp-per-track form of small batches in group_api.cu.  All write the
+// slot-major records of dprop_results.
 #include <cuda_runtime.h>
 
 #include <cub/device/device_radix_sort.cuh>
@@ -268,17 +269,9 @@ __global__ void direction_key_kernel(const In* __restrict__ dx,
 }
 
 
-// Threads per CTA and the minimum resident CTAs per SM the register
-// allocation targets (__launch_bounds__); overridable at build time for
-// tuning sweeps.
+// Threads per CTA; overridable at build time for tuning sweeps.
 #ifndef DPROP_BLOCK
 #define DPROP_BLOCK 128
-#endif
-#ifndef DPROP_MIN_BLOCKS
-// 12 resident CTAs of 128 threads per SM (40 registers per thread): measured
-// on B200 to hide the latency of the divergent navigation better than fewer
-// warps with more registers, despite the extra spills to L1
-#define DPROP_MIN_BLOCKS 12
 #endif
 constexpr int k_plain_block = DPROP_BLOCK;
 // Largest CTA a plain launch may use (dprop_launch.block_size): the kernels
@@ -289,12 +282,12 @@ static_assert(k_plain_max_block % k_plain_block == 0,
               "the largest plain CTA is a multiple of the default one");
 
 // One instantiation per register budget: MinBlocks resident CTAs of 128
-// threads per SM -> 8: 64 registers, 12: 40 registers, 16: 32 registers per
+// threads per SM -> 4: 128 registers, 8: 64, 12: 40, 16: 32 registers per
 // thread (the rest spills to L1).  More resident warps hide more of the
-// navigation's memory and instruction-fetch latency; the best budget depends
-// on the workload (constant field vs field map), so it is a launch choice.
-template <typename In, int MinBlocks = DPROP_MIN_BLOCKS, bool W = true,
-          bool Grad = false>
+// navigation's memory and instruction-fetch latency, fewer spill less; the
+// best budget follows the batch size and the workload (plain_budget,
+// core/launch_rules.hpp; 12 only where a launch names it).
+template <typename In, int MinBlocks, bool W, bool Grad = false>
 __global__ void __launch_bounds__(
     k_plain_max_block, MinBlocks * k_plain_block / k_plain_max_block)
     propagate_plain_kernel(const __grid_constant__ detector_view<float, W> det,
@@ -368,10 +361,8 @@ __global__ void __launch_bounds__(128)
 
 namespace dprop::api {
 
-// register budget of a launch: resident CTAs per SM in {8, 12, 16}
 int occupancy_of(const dprop_launch* lc) {
-    const uint32_t v = (lc && lc->ctas_per_sm) ? lc->ctas_per_sm
-                                               : static_cast<uint32_t>(DPROP_MIN_BLOCKS);
+    const uint32_t v = (lc && lc->ctas_per_sm) ? lc->ctas_per_sm : 12u;
     return v <= 8u ? 8 : (v <= 12u ? 12 : 16);
 }
 

@@ -37,9 +37,9 @@
 // queue is empty.  Once fewer than tail_tracks tracks are alive (the count
 // kernel decides it on the device), they are left to the tail: the phase
 // kernels of the remaining rounds leave at once, and the tail kernels run the
-// tracks to their end with every segment inline.  Records are staged as one 128-byte (fp32) or 256-byte
-// (fp64) row per record and converted to the result layout at the end
-// (rounds_unstage_kernel).  Each kernel loads and stores only the state its
+// tracks to their end with every segment inline.  Records are staged as one
+// 128-byte (fp32) or 256-byte (fp64) row per record and converted to the
+// result layout at the end (rounds_unstage_kernel).  Each kernel loads and stores only the state its
 // segments use; the segments perform the loop's operations in its order,
 // so a track driven through the phases ends as it would in the one-shot
 // loop (bit for bit in a host build of both; on the device the separately
@@ -392,7 +392,7 @@ __global__ void __launch_bounds__(k_phase_block)
 
 // The step phase, compiled for MinBlocks resident CTAs per SM: 3 (168
 // registers: the state and the step's temporaries fit with hardly a spill),
-// 4 (128) or 5 (96).  It waits for loads and instructions, 20 % of its issue
+// 4 (128) or 5 (96).  It waits for loads and instructions, 27-29 % of its issue
 // slots are used; the traffic of spilled state costs more than further warps
 // hide.  B200, 3 / 4 / 5 CTAs, 1.5 M toy tracks: 29.1 / 30.8 / 33.2 ms, in the
 // field map 35.4 / 37.0 / 40.1 ms; with the candidates in registers

@@ -319,9 +319,10 @@ typedef enum dprop_method {
                                     volume switch), in direction order, and
                                     persistent
                                     grid-stride kernels pull their tracks
-                                    from those queues; after `rounds` rounds
-                                    the tracks still alive finish in one
-                                    kernel.  Identical results to the plain
+                                    from those queues; after `rounds` rounds,
+                                    or once few are left (tail_tracks), the
+                                    tracks still alive finish a warp per
+                                    track.  Identical results to the plain
                                     form                                      */
 } dprop_method;
 
@@ -334,15 +335,20 @@ typedef struct dprop_launch {
     uint32_t ctas_per_sm;        /* register budget: resident CTAs of 128
                                     threads per SM the kernel is compiled for.
                                     Plain method: 8 (64 registers), 12 (40)
-                                    or 16 (32); 0 = 12.  Persistent method,
-                                    its step phase: 3 (168 registers), 4
-                                    (128) or 5 (102); 0 = 4.  fp64 plain: 8
-                                    or 12 (0 = 8); fp64 persistent: 2 (255
-                                    registers) or 3 (168); 0 = 2              */
+                                    or 16 (32); 0: by batch size, 4 (128), 8
+                                    or 16.  Persistent method, its step
+                                    phase: 3 (168 registers), 4 (128) or 5
+                                    (96); 0 = 3.  fp64 plain: 8 or 12; 0: by
+                                    batch size, 2 (255), 4 or 8; fp64
+                                    persistent: 2 (255 registers) or 3
+                                    (168); 0 = 2                              */
     uint32_t sort_tracks;        /* 1: process tracks ordered by direction
                                     (theta, phi) so that the lanes of a warp
                                     follow similar paths; results are still
-                                    written at each track's input position    */
+                                    written at each track's input position.
+                                    Left out where the form does not need it
+                                    (a warp per track, small batches of a
+                                    detector with short surface lists)        */
     uint32_t use_graph;          /* 1: capture the whole propagate call into a
                                     CUDA graph on first use and replay it on
                                     later calls with identical arguments       */
@@ -434,7 +440,8 @@ dprop_status dprop_propagate(const dprop_config* cfg,
  * synchronises.  Uses library-owned device scratch, grown on demand.  With
  * jagged records (rec_offsets) the batch runs in chunks of up to 256 Ki
  * tracks on four streams, each chunk with the launch's method, sort and
- * register budget (use_graph is ignored there). */
+ * register budget, or, with the shape left open, in the form of the chunk's
+ * size (use_graph is ignored there). */
 dprop_status dprop_propagate_host(const dprop_config* cfg,
                                   const dprop_launch* launch,
                                   const dprop_detector* det,
@@ -500,12 +507,14 @@ dprop_status dprop_propagate_direct(const dprop_config* cfg,
  * record (a marker at the track origin) is not written.
  *
  * Mask tolerance: mask_tolerance mm on sensitive and passive surfaces, none
- * on portals, as the reference scanner.  The scan is brute force: its cost
- * is n_tracks x n_surfaces root searches. */
+ * on portals, as the reference scanner.  Every surface is tested against the
+ * track's helix (a sphere around planar surfaces); the root search runs for
+ * those it may hit (about 200 of the toy detector's 4 158). */
 typedef enum dprop_scan_status {
     DPROP_SCAN_OK = 0,
     DPROP_SCAN_OVERFLOW = 1,  /* more intersections than capacity: n_hits
-                                 holds the number found, nothing is stored  */
+                                 holds the number found; the arrays hold an
+                                 unsorted part of them                      */
     DPROP_SCAN_EMPTY = 2      /* no intersection at all                     */
 } dprop_scan_status;
 
@@ -640,8 +649,9 @@ dprop_status dprop_detector_info(const dprop_detector* det, uint32_t* n_volumes,
  * start-to-first-surface Jacobian and the derivative of the material
  * interaction's q/p kick.
  *
- * dprop_propagate_adjoint is dprop_propagate (plain kernel; launch->method and
- * use_graph are ignored) plus a tape of derivative data:
+ * dprop_propagate_adjoint is dprop_propagate (plain kernel, a warp per track
+ * for small batches with an open shape; launch->method and use_graph are
+ * ignored) plus a tape of derivative data:
  *   tape->rec:  float [DPROP_TAPE_RECORD_FLOATS][max_records][n]
  *   tape->init: float [DPROP_TAPE_TRACK_FLOATS][n]
  * (device memory, written for every stored transported record and every
