@@ -573,8 +573,10 @@ struct launch_plan {
 // sorted track's record, written field by field at its input index, touches
 // 31 sectors for 121 bytes.  Smaller batches stay in L2, which merges them.
 // B200, us, staged against direct: toy 16 384: 1 111 / 1 284, 150 000: 3 641 /
-// 3 921, 1 000 000: 20 814 / 23 569; the telescope 1 200 000 in input order
-// 7 649, sorted and staged 6 448.
+// 3 921, 1 000 000: 20 814 / 23 569; wire chamber 16 384: 2 979 / 3 193, 100 000:
+// 7 840 / 8 168 (12 000: 2 991 / 2 905); toy with material maps 16 384: 1 564 /
+// 1 766; telescope 16 384: 363 / 384, 1 200 000 in input order 7 649, sorted and
+// staged 6 448.
 constexpr uint64_t k_stage_from = 16384u;
 // The staging area is kept between calls, so it is bounded: larger batches
 // write directly.
