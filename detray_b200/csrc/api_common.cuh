@@ -148,6 +148,7 @@ struct dprop_detector {
     // include the code for them
     bool wires{false};
     dprop::launch_traits traits;
+    uint32_t n_unbounded{0};  // surfaces the truth scan searches for any track
     dprop::detector_view<double> view_d() const { return view_d_as<true>(); }
     template <bool W>
     dprop::detector_view<double, W> view_d_as() const {

@@ -183,6 +183,15 @@ inline int plain_budget(const launch_traits& t, bool field_map,
     return field_map && t.surface_grids && tracks_per_sm >= 1536u ? 16 : 8;
 }
 
+// Whether the truth scan of n tracks runs a cluster of eight CTAs per track:
+// unbounded is the number of surfaces the culling cannot skip (cylinders and
+// lines), 256 the threads of a CTA.  Wire chamber, one CTA / a cluster: 1 track
+// 250 / 83, 128: 255 / 159, 192: 280 / 202, 1 000: 721 / 771; fp64 1: 333 / 90,
+// 192: 383 / 340, 256: 385 / 437.
+inline bool scan_in_clusters(uint32_t unbounded, uint64_t n) {
+    return unbounded > 256u && n <= 192u;
+}
+
 // Device scratch of a host call without jagged records: inputs (8 doubles a
 // track), per-track outputs (status, six counters, path length, the 8 final
 // parameters) and records (barcode, 6 + 21 + 1 floats, flags), each array

@@ -1438,6 +1438,10 @@ dprop_status dprop_detector_create(const dprop_detector_desc* d, int device,
     det->device = device;
     det->n_volumes = d->n_volumes;
     det->n_surfaces = d->n_surfaces;
+    const std::vector<scan_bound> bounds = scan_bounds(d);
+    for (const scan_bound& b : bounds) {
+        det->n_unbounded += b.radius < 0.f ? 1u : 0u;
+    }
     dprop_status st = DPROP_OK;
     if ((st = upload(t.volumes, &det->volumes)) != DPROP_OK ||
         (st = upload(t.surfaces, &det->surfaces)) != DPROP_OK ||
@@ -1448,7 +1452,7 @@ dprop_status dprop_detector_create(const dprop_detector_desc* d, int device,
         (st = upload(t.bf_surfaces, &det->bf_surfaces)) != DPROP_OK ||
         (st = upload(t.grids, &det->grids)) != DPROP_OK ||
         (st = upload(t.grid_bins, &det->grid_bins)) != DPROP_OK ||
-        (st = upload(scan_bounds(d), &det->scan_bounds)) != DPROP_OK ||
+        (st = upload(bounds, &det->scan_bounds)) != DPROP_OK ||
         (!t.vol_material.empty() &&
          (st = upload(t.vol_material, &det->vol_material)) != DPROP_OK)) {
         dprop_detector_destroy(det);

@@ -2,7 +2,7 @@
 // dprop_helix_scan and dprop_validate_navigation (dprop.h).
 //
 // Kernels:
-//   helix_scan_kernel    one CTA per track: the surfaces are tested against
+//   helix_scan_kernel    one CTA (or a cluster) per track: the surfaces are tested against
 //                        the track's helix (scan_may_hit, core/helix.cuh) and
 //                        the few it may hit are intersected (root search,
 //                        one thread per surface); hits inside a mask and
@@ -13,7 +13,10 @@
 //   validate_kernel      one thread per track: holes and extra surfaces of
 //                        a propagation's records against the scan
 // The surfaces of a detector are read by every track: they stay in L2.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
+
+#include <type_traits>
 
 #include "api_common.cuh"
 #include "core/helix.cuh"
@@ -23,7 +26,15 @@ using dprop::api::fail;
 
 namespace {
 
-constexpr int k_scan_block = 256;  // a track's surfaces to search: one pass
+// Threads of a track's CTA: most tracks' surfaces to search take one pass.
+constexpr int k_scan_block = 256;
+// Of a detector with no more surfaces than a warp has lanes: more warps would
+// only be launched and wait at the barriers (telescope, field across it, 4 000
+// tracks 158 us with 256 threads, 84 with 32; in double 1 000: 134 / 75).
+constexpr int k_scan_block_few = 32;
+// CTAs of a track's cluster where few tracks have many surfaces to search.
+constexpr int k_scan_cluster = 8;
+constexpr int k_validate_block = 256;
 
 template <typename S>
 struct scan_io {
@@ -132,20 +143,35 @@ __device__ uint32_t finish_in_results(const scan_io<S>& io, uint64_t t,
 // against 2.18 ms).  8 192 toy tracks in fp32: 99.2 ms with a search per
 // (track, surface), 2.0 ms now; 1 500 tracks in fp64 with the propagation
 // they validate: 155.6 ms before, 3.0 ms now (B200).
-template <typename S, bool W>
-__global__ void __launch_bounds__(k_scan_block)
+//
+// Block: threads of a CTA.  Ctas > 1: a cluster of that many per track divides
+// the surfaces and collects the hits in its first CTA's shared memory.  Few
+// tracks leave SMs idle, and the culling keeps every cylinder and line of a
+// wire chamber (1 933 surfaces: eight passes of searches, one after the other;
+// one track 250 us in one CTA, 83 in a cluster, in double 333 and 90).
+template <typename S, bool W, int Block, int Ctas>
+__global__ void __launch_bounds__(Block)
     helix_scan_kernel(const __grid_constant__ detector_view<S, W> det,
                       const scan_bound* __restrict__ bounds,
                       const __grid_constant__ scan_io<S> io, vec3<S> bfield,
                       S mask_tol, uint64_t n) {
-    __shared__ hit_list<S> hits;
-    __shared__ uint32_t todo[2 * k_scan_block];
-    __shared__ uint32_t n_todo, n_found, n_kept;
-    const uint64_t t = blockIdx.x;
+    __shared__ hit_list<S> own_hits;
+    __shared__ uint32_t todo[2 * Block];
+    __shared__ uint32_t n_todo, own_found, n_kept;
+    const uint64_t t = blockIdx.x / static_cast<uint32_t>(Ctas);
+    const uint32_t part = blockIdx.x % static_cast<uint32_t>(Ctas);
     const uint32_t tid = threadIdx.x;
+    hit_list<S>* all_hits = &own_hits;
+    uint32_t* n_found = &own_found;
+    if constexpr (Ctas > 1) {
+        const auto cluster = cooperative_groups::this_cluster();
+        all_hits = cluster.map_shared_rank(&own_hits, 0);
+        n_found = cluster.map_shared_rank(&own_found, 0);
+    }
+    hit_list<S>& hits = *all_hits;
     if (tid == 0u) {
         n_todo = 0u;
-        n_found = 0u;
+        own_found = 0u;
     }
     helix<S> h;
     h.init(vec3<S>{io.trk[0][t], io.trk[1][t], io.trk[2][t]},
@@ -156,8 +182,14 @@ __global__ void __launch_bounds__(k_scan_block)
     const float tol = static_cast<float>(mask_tol);
     const root_cfg<S> cfg{S(unit::um), 1000u, S(5000) * S(unit::mm)};
     const uint32_t cap = io.capacity;
-    __syncthreads();
-    for (uint32_t base = 0u; base < det.n_surfaces; base += k_scan_block) {
+    if constexpr (Ctas > 1) {
+        // the first CTA's counter is set, and its shared memory there
+        cooperative_groups::this_cluster().sync();
+    } else {
+        __syncthreads();
+    }
+    constexpr uint32_t stride = Ctas * Block;
+    for (uint32_t base = part * Block; base < det.n_surfaces; base += stride) {
         const uint32_t sf = base + tid;
         const bool keep =
             sf < det.n_surfaces && scan_may_hit(bounds[sf], probe, tol);
@@ -174,15 +206,15 @@ __global__ void __launch_bounds__(k_scan_block)
         uint32_t m = n_todo;
         __syncthreads();  // every thread has read it
         // a full CTA of surfaces, or the last ones
-        const bool last = base + k_scan_block >= det.n_surfaces;
-        const bool search = m >= k_scan_block || (last && m > 0u);
-        while (m >= k_scan_block || (last && m > 0u)) {
-            const uint32_t first = m > k_scan_block ? m - k_scan_block : 0u;
+        const bool last = base + stride >= det.n_surfaces;
+        const bool search = m >= Block || (last && m > 0u);
+        while (m >= Block || (last && m > 0u)) {
+            const uint32_t first = m > Block ? m - Block : 0u;
             if (first + tid < m) {
                 helix_surface_hits(
                     det, todo[first + tid], h, mask_tol, cfg,
                     [&](const scan_hit<S>& hit) {
-                        const uint32_t k = atomicAdd(&n_found, 1u);
+                        const uint32_t k = atomicAdd(n_found, 1u);
                         const uint64_t bc = det.surfaces[hit.sf].barcode;
                         if (k < k_smem_hits) {
                             hits.path[k] = hit.path;
@@ -207,7 +239,14 @@ __global__ void __launch_bounds__(k_scan_block)
             __syncthreads();
         }
     }
-    const uint32_t found = n_found;
+    if constexpr (Ctas > 1) {
+        // every CTA's hits are in the first one's list, which goes on alone
+        cooperative_groups::this_cluster().sync();
+        if (part != 0u) {
+            return;
+        }
+    }
+    const uint32_t found = own_found;
     if (found == 0u) {
         if (tid == 0u) {
             io.n_hits[t] = 0u;
@@ -221,7 +260,7 @@ __global__ void __launch_bounds__(k_scan_block)
     __syncthreads();
     const bool in_smem = found <= k_smem_hits && found <= cap;
     const uint32_t held = found < k_smem_hits ? found : k_smem_hits;
-    for (uint32_t k = tid; k < held; k += k_scan_block) {
+    for (uint32_t k = tid; k < held; k += Block) {
         uint32_t slot = k;
         if (in_smem) {
             // the hit's place in the sorted list
@@ -279,34 +318,53 @@ dprop_status launch_scan(const dprop_detector* det, const double b[3],
     io.capacity = r->capacity;
     const vec3<S> bf{static_cast<S>(b[0]), static_cast<S>(b[1]),
                      static_cast<S>(b[2])};
-    const unsigned int grid = static_cast<unsigned int>(n);
+    const auto run = [&](auto view) -> dprop_status {
+        using view_t = decltype(view);
+        constexpr bool W =
+            std::is_same<view_t, detector_view<S, true>>::value;
+        cudaLaunchConfig_t lc{};
+        lc.stream = st;
+        lc.gridDim = dim3(static_cast<unsigned int>(n));
+        lc.blockDim = dim3(k_scan_block);
+        cudaLaunchAttribute cluster{};
+        const S tol = static_cast<S>(mask_tol);
+        if (det->n_surfaces <= static_cast<uint32_t>(k_scan_block_few)) {
+            lc.blockDim = dim3(k_scan_block_few);
+            DPROP_CUDA(cudaLaunchKernelEx(
+                &lc, helix_scan_kernel<S, W, k_scan_block_few, 1>, view,
+                static_cast<const scan_bound*>(det->scan_bounds), io, bf, tol,
+                n));
+        } else if (scan_in_clusters(det->n_unbounded, n)) {
+            lc.gridDim = dim3(static_cast<unsigned int>(n * k_scan_cluster));
+            cluster.id = cudaLaunchAttributeClusterDimension;
+            cluster.val.clusterDim.x = k_scan_cluster;
+            cluster.val.clusterDim.y = 1;
+            cluster.val.clusterDim.z = 1;
+            lc.attrs = &cluster;
+            lc.numAttrs = 1;
+            DPROP_CUDA(cudaLaunchKernelEx(
+                &lc, helix_scan_kernel<S, W, k_scan_block, k_scan_cluster>,
+                view, static_cast<const scan_bound*>(det->scan_bounds), io, bf,
+                tol, n));
+        } else {
+            DPROP_CUDA(cudaLaunchKernelEx(
+                &lc, helix_scan_kernel<S, W, k_scan_block, 1>, view,
+                static_cast<const scan_bound*>(det->scan_bounds), io, bf, tol,
+                n));
+        }
+        return DPROP_OK;
+    };
     if constexpr (sizeof(S) == 8) {
-        if (det->wires) {
-            helix_scan_kernel<S, true><<<grid, k_scan_block, 0, st>>>(
-                det->view_d_as<true>(), det->scan_bounds, io, bf,
-                static_cast<S>(mask_tol), n);
-        } else {
-            helix_scan_kernel<S, false><<<grid, k_scan_block, 0, st>>>(
-                det->view_d_as<false>(), det->scan_bounds, io, bf,
-                static_cast<S>(mask_tol), n);
-        }
+        return det->wires ? run(det->view_d_as<true>())
+                          : run(det->view_d_as<false>());
     } else {
-        if (det->wires) {
-            helix_scan_kernel<S, true><<<grid, k_scan_block, 0, st>>>(
-                det->view_as<true>(), det->scan_bounds, io, bf,
-                static_cast<S>(mask_tol), n);
-        } else {
-            helix_scan_kernel<S, false><<<grid, k_scan_block, 0, st>>>(
-                det->view_as<false>(), det->scan_bounds, io, bf,
-                static_cast<S>(mask_tol), n);
-        }
+        return det->wires ? run(det->view_as<true>())
+                          : run(det->view_as<false>());
     }
-    DPROP_CUDA(cudaGetLastError());
-    return DPROP_OK;
 }
 
 template <typename Ti, typename Tr>
-__global__ void __launch_bounds__(k_scan_block)
+__global__ void __launch_bounds__(k_validate_block)
     validate_kernel(const uint8_t* __restrict__ scan_status,
                     const uint32_t* __restrict__ n_hits,
                     const uint64_t* __restrict__ truth_bc,
@@ -338,8 +396,8 @@ void launch_validate(const dprop_scan_results* s, const dprop_results* r,
                      uint32_t max_records, uint64_t n, double tol,
                      const dprop_validation* out, cudaStream_t st) {
     const unsigned int tb =
-        static_cast<unsigned int>((n + k_scan_block - 1) / k_scan_block);
-    validate_kernel<Ti, Tr><<<tb, k_scan_block, 0, st>>>(
+        static_cast<unsigned int>((n + k_validate_block - 1) / k_validate_block);
+    validate_kernel<Ti, Tr><<<tb, k_validate_block, 0, st>>>(
         s->status, s->n_hits, s->barcode, static_cast<const Ti*>(s->path),
         s->volume_link, r->status, r->n_records, r->rec_barcode,
         static_cast<const Tr*>(r->rec_path), max_records, n, tol,

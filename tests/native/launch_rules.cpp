@@ -18,6 +18,14 @@ extern "C" uint64_t host_scratch(uint64_t n, uint64_t max_records) {
     return host_scratch_bytes(n, max_records);
 }
 
+extern "C" int scan_clusters(const dprop_detector_desc* d, uint64_t n) {
+    uint32_t unbounded = 0u;
+    for (const scan_bound& b : scan_bounds(d)) {
+        unbounded += b.radius < 0.f ? 1u : 0u;
+    }
+    return scan_in_clusters(unbounded, n) ? 1 : 0;
+}
+
 extern "C" int drops_order(const dprop_detector_desc* d, int staged,
                            uint64_t n) {
     return order_is_a_loss(launch_traits_of(d, false), staged != 0, n) ? 1 : 0;

@@ -46,6 +46,11 @@ def rules(tmp_path_factory):
     lib.host_scratch.restype = C.c_uint64
     get.host_scratch = lambda n, r: lib.host_scratch(C.c_uint64(n),
                                                      C.c_uint64(r))
+    def scan_clusters(tables, n):
+        desc = geometry.Descriptor(tables)
+        return bool(lib.scan_clusters(C.byref(desc.desc), C.c_uint64(n)))
+
+    get.scan_clusters = scan_clusters
     get.budget = budget
     get.drops_order = drops_order
     get.load = geometry.load_geometry
@@ -172,3 +177,12 @@ def test_host_scratch_holds_every_array(rules, n, max_records):
     for s in sizes:
         end += -(-s // 256) * 256
     assert rules.host_scratch(n, max_records) >= end
+
+
+def test_scan_of_few_tracks(rules):
+    """Few tracks of a detector whose surfaces the truth scan cannot skip."""
+    wire = rules.load("wire_chamber_10l_cells")
+    assert rules.scan_clusters(wire, 1) and rules.scan_clusters(wire, 100)
+    assert not rules.scan_clusters(wire, 1000)
+    assert not rules.scan_clusters(rules.load("toy_4brl_7edc"), 1)
+    assert not rules.scan_clusters(rules.load("telescope_10x1m_300um"), 1)
