@@ -217,7 +217,8 @@ dprop_status dprop_propagate_adjoint(const dprop_config* cfg,
     DPROP_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     const uint64_t per_sm = n / static_cast<uint64_t>(sms);
     if (api::open_shape(lc) &&
-        n <= group_limit_adjoint(det->traits, pc.step.field_gradient)) {
+        n <= group_limit_adjoint(det->traits, cfg->search_window,
+                                 pc.step.field_gradient)) {
         if (!pc.step.field_gradient) {
             launch_adjoint_group<16, false>(st, det, field->view, pc, io, tv,
                                             n);

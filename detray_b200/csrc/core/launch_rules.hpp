@@ -42,6 +42,19 @@ inline launch_traits launch_traits_of(const dprop_detector_desc* d,
     return t;
 }
 
+// Bins of a grid that a search looks at, with the configuration's window.
+inline uint64_t window_bins(const uint32_t window[2]) {
+    const uint64_t side = uint64_t(window[0]) + window[1] + 1u;
+    return side * side;
+}
+
+// Whether a search of that window is a small part of a track: the lanes of a
+// warp have little to share, and more warps per SM little to hide.
+inline bool narrow_search(const launch_traits& t, const uint32_t window[2]) {
+    return t.surface_grids &&
+           window_bins(window) < (t.extra_code ? 16u : 9u);
+}
+
 // Tracks up to which a warp per track is the faster form, fp32.  The lanes of a
 // warp share only the searches, so beyond a full GPU one thread per track
 // wins; how far beyond depends on how much of a track is search.  Warp per
@@ -56,6 +69,11 @@ inline launch_traits launch_traits_of(const dprop_detector_desc* d,
 //   telescope (no grid, 11 surfaces) 2 300: 215 / 249 / 307, 3 000: 340 / 248 /
 //   308; with volume material 1 400: 305 / 322 / 384, 1 800: 328 / 316 / 389,
 //   10 000: 1 669 / 347 / 430
+// all with windows of 3 bins either side.  With a window of one bin, half the
+// limit, a warp / a thread per track:
+//   toy 4 000: 588 / 581, 6 000: 874 / 581; with material maps 2 000: 778 / 757,
+//   4 000: 1 198 / 757 (3 x 3 bins 2 000: 994 / 1 197); wire chamber in the map
+//   5 000: 1 928 / 1 775, 8 000: 2 906 / 1 983
 inline uint64_t group_limit(const launch_traits& t) {
     if (t.lines) {
         return 8192u;
@@ -64,6 +82,9 @@ inline uint64_t group_limit(const launch_traits& t) {
         return t.extra_code ? 4096u : 6144u;
     }
     return t.extra_code ? 1536u : 2368u;
+}
+inline uint64_t group_limit(const launch_traits& t, const uint32_t window[2]) {
+    return group_limit(t) / (narrow_search(t, window) ? 2u : 1u);
 }
 
 // The same in the adjoint propagation.  It pays for fewer tracks there: the
@@ -78,9 +99,19 @@ inline uint64_t group_limit(const launch_traits& t) {
 //   material maps 2 300: 1 491 / 2 403 / 1 835, 3 000: 2 051 / 2 425 / 1 774;
 //   wire chamber 5 000: 3 100 / 2 799 / 2 962 (pT from 0.1 GeV 3 843 / 8 274 /
 //   8 223); telescope 1 400: 345 / 384 / 455, 3 000: 537 / 396 / 472
+// The window matters to the form without the field gradient alone (one bin:
+// toy 2 700: 716 / 780, 4 000: 961 / 780; with it the searches are a small part
+// anyway), and a window of 3 x 3 bins only where there are lines (wire chamber
+// in the map 5 400: 3 664 / 3 258).
 inline uint64_t group_limit_adjoint(const launch_traits& t,
+                                    const uint32_t window[2],
                                     bool field_gradient) {
-    return field_gradient ? group_limit(t) / 4u : 2u * group_limit(t) / 3u;
+    if (field_gradient) {
+        return group_limit(t) / 4u;
+    }
+    const bool narrow = t.surface_grids &&
+                        window_bins(window) < (t.lines ? 16u : 9u);
+    return 2u * group_limit(t) / (narrow ? 6u : 3u);
 }
 
 // The same in double precision.  Warp per track / thread per track / sorted:
@@ -89,13 +120,17 @@ inline uint64_t group_limit_adjoint(const launch_traits& t,
 // 2 501 / 1 889; wire chamber 4 000: 2 969 / 2 840 / 2 879, 5 000: 3 649 / 2 891 /
 // 2 972 (pT from 0.1 GeV 4 640 / 8 960 / 8 862); telescope 1 000: 217 / 288 /
 // 355, 1 800: 333 / 289 / 353; with volume material 1 000: 326 / 411 / 478,
-// 1 400: 529 / 425 / 483, 8 000: 2 206 / 436 / 527.
-inline uint64_t group_limit_fp64(const launch_traits& t) {
+// 1 400: 529 / 425 / 483, 8 000: 2 206 / 436 / 527.  With a window of one bin:
+// toy 2 000: 584 / 665, 3 000: 862 / 665; with material maps 1 000: 814 / 966,
+// 3 000: 1 884 / 966.
+inline uint64_t group_limit_fp64(const launch_traits& t,
+                                 const uint32_t window[2]) {
+    const uint64_t part = narrow_search(t, window) ? 2u : 1u;
     if (t.lines) {
-        return 5120u;
+        return 5120u / part;
     }
     if (t.surface_grids) {
-        return 3072u;
+        return 3072u / part;
     }
     return t.extra_code ? 1184u : 2048u;
 }
@@ -163,11 +198,13 @@ inline bool order_is_a_loss(const launch_traits& t, bool staged, uint64_t n) {
 // Register budget of the plain kernel, fp32: resident CTAs of 128 threads per
 // SM, 4 (128 registers) while that keeps the whole batch resident, 512 tracks
 // per SM; else 8 (64).  In a field map 16 (32 registers) from 1 536 per SM on
-// when the volumes have surface grids: more warps hide the lookups and the
-// grid's loads.  Tracks that test a list have less to hide.  4 / 8 / 12 / 16:
+// when the volumes have surface grids and the window is wide: more warps hide
+// the lookups and the grid's loads.  Tracks that test a list or one bin have
+// less to hide.  4 / 8 / 12 / 16:
 //   toy 75 000: 2 532 / 2 742 / 3 210 / 3 526, 150 000: 4 847 / 3 710 / 4 770 /
 //   4 972, 1 200 000: - / 25 022 / 27 294 / 25 483; in the map 150 000: 7 772 /
-//   6 169 / 7 846 / 8 051, 300 000: - / 11 694 / 13 054 / 10 778
+//   6 169 / 7 846 / 8 051, 300 000: - / 11 694 / 13 054 / 10 778; with a window
+//   of one bin 450 000: - / 7 111 / 8 181 / 9 599
 //   wire chamber in the map 300 000: - / 19 504 / 23 051 / 17 542; toy with
 //   material maps in the map 300 000: - / 12 556 / 13 829 / 11 860
 //   telescope 10 000: 234 / 276 / 317 / 347; in the map 300 000: - / 2 051 /
@@ -175,12 +212,15 @@ inline bool order_is_a_loss(const launch_traits& t, bool staged, uint64_t n) {
 //   the toy detector's modules as lists (1 096 in a volume), in the map, input
 //   order 230 000: 49 412 / 28 715 / 34 391 / 34 001, sorted 25 674 / 18 328 /
 //   18 072 / 22 662
-inline int plain_budget(const launch_traits& t, bool field_map,
-                        uint64_t tracks_per_sm) {
+inline int plain_budget(const launch_traits& t, const uint32_t window[2],
+                        bool field_map, uint64_t tracks_per_sm) {
     if (tracks_per_sm < 512u) {
         return 4;
     }
-    return field_map && t.surface_grids && tracks_per_sm >= 1536u ? 16 : 8;
+    return field_map && t.surface_grids && window_bins(window) >= 16u &&
+                   tracks_per_sm >= 1536u
+               ? 16
+               : 8;
 }
 
 // Whether the truth scan of n tracks runs a cluster of eight CTAs per track:

@@ -473,8 +473,8 @@ int plain_block_of(const dprop_launch* lc) {
 
 // Register budget of a plain launch, the spelled-out one or plain_budget's.
 dprop_status launch_budget(const dprop_launch* lc, const dprop_detector* det,
-                           const field_view<float>& field, uint64_t n,
-                           int* mb) {
+                           const field_view<float>& field,
+                           const prop_cfg<float>& cfg, uint64_t n, int* mb) {
     *mb = occupancy_of(lc);
     if (lc && lc->ctas_per_sm) {
         return DPROP_OK;
@@ -482,7 +482,8 @@ dprop_status launch_budget(const dprop_launch* lc, const dprop_detector* det,
     int dev = 0, sms = 0;
     DPROP_CUDA(cudaGetDevice(&dev));
     DPROP_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    *mb = plain_budget(det->traits, field.kind != 0u,
+    const uint32_t window[2] = {cfg.nav.win0, cfg.nav.win1};
+    *mb = plain_budget(det->traits, window, field.kind != 0u,
                        n / static_cast<uint64_t>(sms));
     return DPROP_OK;
 }
@@ -503,7 +504,7 @@ dprop_status launch_plain(const dprop_launch* lc, cudaStream_t st,
                     "256");
     }
     int mb = 0;
-    const dprop_status s = launch_budget(lc, det, field, n, &mb);
+    const dprop_status s = launch_budget(lc, det, field, cfg, n, &mb);
     if (s != DPROP_OK) {
         return s;
     }
@@ -590,7 +591,7 @@ launch_plan plan_launch(const dprop_config& c, const dprop_launch* lc,
                         size_t stage_limit = k_stage_limit) {
     launch_plan p{};
     const bool fg = c.use_field_gradient != 0;
-    p.group = dprop::api::use_group(lc, det, fg, n);
+    p.group = dprop::api::use_group(lc, det, c, n);
     if (p.group) {
         return p;
     }
@@ -2035,7 +2036,7 @@ extern "C" dprop_status dprop_propagate_noalloc(const dprop_config* cfg,
     }
     const io_ptrs<float> io = make_io<float>(*tracks, *results);
     const prop_cfg<float> pc = make_prop_cfg<float>(*cfg);
-    if (dprop::api::use_group(nullptr, det, pc.step.field_gradient, n)) {
+    if (dprop::api::use_group(nullptr, det, *cfg, n)) {
         return dprop::api::enqueue_group<float>(det, field, pc, io, n, stream);
     }
     const int ni = static_cast<int>(n);

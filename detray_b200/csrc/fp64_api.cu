@@ -79,7 +79,7 @@ dprop_status propagate_fp64(const dprop_config& c, const dprop_launch* lc,
     DPROP_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     const uint64_t per_sm = n / static_cast<uint64_t>(sms);
     const bool open = open_shape(lc) && c.use_field_gradient == 0;
-    if (open && n <= group_limit_fp64(det->traits)) {
+    if (open && n <= group_limit_fp64(det->traits, c.search_window)) {
         auto go = [&](auto view) {
             constexpr bool W =
                 std::is_same<decltype(view), detector_view<double, true>>::value;

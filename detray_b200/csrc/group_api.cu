@@ -89,9 +89,10 @@ bool open_shape(const dprop_launch* lc) {
 }
 
 bool use_group(const dprop_launch* lc, const dprop_detector* det,
-               bool field_gradient, uint64_t n) {
+               const dprop_config& cfg, uint64_t n) {
     // a launch shape that is spelled out is launched as it is
-    return open_shape(lc) && !field_gradient && n <= group_limit(det->traits);
+    return open_shape(lc) && cfg.use_field_gradient == 0 &&
+           n <= group_limit(det->traits, cfg.search_window);
 }
 
 template <typename In>

@@ -245,7 +245,7 @@ __device__ __forceinline__ void run_group(uint64_t t, uint64_t n,
 // per track (either method, when the launch leaves its shape open), and the
 // enqueue of that form (no scratch, no order: every track has its own warp).
 bool use_group(const dprop_launch* lc, const dprop_detector* det,
-               bool field_gradient, uint64_t n);
+               const dprop_config& cfg, uint64_t n);
 // Runs every fp32 kernel of that form on no track: the driver loads its code
 // and reserves its local memory now, not at the first call that takes it.
 dprop_status load_group_forms(cudaStream_t stream);

@@ -7,9 +7,10 @@ using namespace dprop;
 // extra_code: as the library finds it (line surfaces, rods, multi-entry bins,
 // material maps, volume material)
 extern "C" int plain_budget_of(const dprop_detector_desc* d, int extra_code,
-                               int field_map, uint64_t tracks_per_sm) {
-    return plain_budget(launch_traits_of(d, extra_code != 0), field_map != 0,
-                        tracks_per_sm);
+                               const uint32_t* window, int field_map,
+                               uint64_t tracks_per_sm) {
+    return plain_budget(launch_traits_of(d, extra_code != 0), window,
+                        field_map != 0, tracks_per_sm);
 }
 
 extern "C" uint32_t tail_of(uint64_t n) { return default_tail_tracks(n); }
@@ -32,15 +33,16 @@ extern "C" int drops_order(const dprop_detector_desc* d, int staged,
 }
 
 extern "C" int launch_rules(const dprop_detector_desc* d, int extra_code,
-                            int field_map, uint64_t* out) {
+                            const uint32_t* window, int field_map,
+                            uint64_t* out) {
     if (!validate_desc(d).empty()) {
         return 1;
     }
     const launch_traits t = launch_traits_of(d, extra_code != 0);
-    out[0] = group_limit(t);
-    out[1] = group_limit_fp64(t);
-    out[2] = group_limit_adjoint(t, false);
-    out[3] = group_limit_adjoint(t, true);
+    out[0] = group_limit(t, window);
+    out[1] = group_limit_fp64(t, window);
+    out[2] = group_limit_adjoint(t, window, false);
+    out[3] = group_limit_adjoint(t, window, true);
     out[4] = rounds_from(t, field_map != 0);
     out[5] = rounds_from_fp64(t);
     return 0;

@@ -24,18 +24,20 @@ def rules(tmp_path_factory):
                     "-o", str(out)], check=True)
     lib = C.CDLL(str(out))
 
-    def get(tables, extra_code, field_map=0):
+    def get(tables, extra_code, field_map=0, window=3):
         desc = geometry.Descriptor(tables)
         v = (C.c_uint64 * 6)()
-        assert lib.launch_rules(C.byref(desc.desc), extra_code, field_map,
+        w = (C.c_uint32 * 2)(window, window)
+        assert lib.launch_rules(C.byref(desc.desc), extra_code, w, field_map,
                                 v) == 0
         return dict(zip(("group", "group64", "adjoint", "adjoint_grad",
                          "rounds", "rounds64"), v))
 
-    def budget(tables, extra_code, field_map, tracks_per_sm):
+    def budget(tables, extra_code, field_map, tracks_per_sm, window=3):
         desc = geometry.Descriptor(tables)
-        return lib.plain_budget_of(C.byref(desc.desc), extra_code, field_map,
-                                   C.c_uint64(tracks_per_sm))
+        w = (C.c_uint32 * 2)(window, window)
+        return lib.plain_budget_of(C.byref(desc.desc), extra_code, w,
+                                   field_map, C.c_uint64(tracks_per_sm))
 
     def drops_order(tables, staged, n):
         desc = geometry.Descriptor(tables)
@@ -186,3 +188,22 @@ def test_scan_of_few_tracks(rules):
     assert not rules.scan_clusters(wire, 1000)
     assert not rules.scan_clusters(rules.load("toy_4brl_7edc"), 1)
     assert not rules.scan_clusters(rules.load("telescope_10x1m_300um"), 1)
+
+
+def test_narrow_windows(rules):
+    """With a window of one bin the searches are a small part of a track: the
+    warp-per-track form ends earlier, and 32 registers do not pay."""
+    toy, maps, wire, tele = (rules.load(x) for x in (
+        "toy_4brl_7edc", "toy_4brl_7edc_maps", "wire_chamber_10l_cells",
+        "telescope_10x1m_300um"))
+    assert 2500 <= rules(toy, 0, 0, 0)["group"] <= 4000
+    assert rules(maps, 1, 0, 0)["group"] <= 2200
+    assert rules(maps, 1, 0, 1)["group"] <= 2500
+    assert rules(wire, 1, 0, 0)["group"] <= 5000
+    assert rules(toy, 0, 0, 0)["group64"] <= 2200
+    assert rules(maps, 1, 0, 0)["group64"] <= 1600
+    # a detector without grids has no window
+    assert rules(tele, 0, 0, 0) == rules(tele, 0, 0, 3)
+    assert rules(toy, 0, 0, 2**32 - 1) == rules(toy, 0, 0, 3)
+    for tables, extra in ((toy, 0), (maps, 1), (wire, 1)):
+        assert rules.budget(tables, extra, 1, 3000, window=0) == 8
