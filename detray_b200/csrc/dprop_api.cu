@@ -1927,9 +1927,12 @@ static __device__ __align__(256) unsigned char
     g_noalloc_scratch[DPROP_NOALLOC_SCRATCH_BYTES];
 
 // Every kernel the entry point may choose by detector, configuration and batch
-// size, run on no track: the driver loads a kernel's code, and reserves the
-// local memory it needs, at its first launch - which would otherwise be an
-// allocation in the middle of a run, at the first batch of another size.
+// size: the driver loads a kernel's code, and reserves the local memory it
+// needs, at its first launch - which would otherwise be an allocation in the
+// middle of a run, at the first batch of another size.  The one-thread-per-track
+// kernels are run on no track, which reserves the most local memory; the
+// others are only loaded (a check for an empty batch in them cost 1 % of a small
+// event).
 template <int MB, bool Grad>
 void launch_empty_plain(cudaStream_t st) {
     const field_view<float> field{};
@@ -1948,7 +1951,7 @@ dprop_status load_noalloc_forms(cudaStream_t st) {
     launch_empty_plain<16, false>(st);
     launch_empty_plain<8, true>(st);
     DPROP_CUDA(cudaGetLastError());
-    return dprop::api::load_group_forms(st);
+    return dprop::api::load_group_forms();
 }
 
 constexpr int k_noalloc_max_devices = 64;

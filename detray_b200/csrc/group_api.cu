@@ -27,10 +27,8 @@ __global__ void __launch_bounds__(32, MinBlocks)
                            const __grid_constant__ prop_cfg<float> cfg,
                            const __grid_constant__ api::io_ptrs<In> io,
                            uint64_t n) {
-    if (blockIdx.x < n) {
-        api::run_group<In>(blockIdx.x, n, det, field, cfg, io,
-                           lane_group<32>::make(threadIdx.x));
-    }
+    api::run_group<In>(blockIdx.x, n, det, field, cfg, io,
+                       lane_group<32>::make(threadIdx.x));
 }
 
 template <int MinBlocks, typename In>
@@ -47,26 +45,21 @@ void launch_group(cudaStream_t st, const dprop_detector* det,
     }
 }
 
-template <int MinBlocks>
-void launch_empty_group(cudaStream_t st) {
-    const field_view<float> field{};
-    const prop_cfg<float> cfg{};
-    const api::io_ptrs<float> io{};
-    propagate_group_kernel<float, true, MinBlocks><<<1, 32, 0, st>>>(
-        detector_view<float, true>{}, field, cfg, io, 0u);
-    propagate_group_kernel<float, false, MinBlocks><<<1, 32, 0, st>>>(
-        detector_view<float, false>{}, field, cfg, io, 0u);
-}
-
 }  // namespace
 
 namespace dprop::api {
 
-dprop_status load_group_forms(cudaStream_t st) {
-    launch_empty_group<16>(st);
-    launch_empty_group<20>(st);
-    launch_empty_group<32>(st);
-    DPROP_CUDA(cudaGetLastError());
+dprop_status load_group_forms() {
+    cudaFuncAttributes a{};
+    const auto load = [&a](auto kernel) {
+        return cudaFuncGetAttributes(&a, kernel);
+    };
+    DPROP_CUDA(load(propagate_group_kernel<float, true, 16>));
+    DPROP_CUDA(load(propagate_group_kernel<float, true, 20>));
+    DPROP_CUDA(load(propagate_group_kernel<float, true, 32>));
+    DPROP_CUDA(load(propagate_group_kernel<float, false, 16>));
+    DPROP_CUDA(load(propagate_group_kernel<float, false, 20>));
+    DPROP_CUDA(load(propagate_group_kernel<float, false, 32>));
     return DPROP_OK;
 }
 

@@ -246,9 +246,9 @@ __device__ __forceinline__ void run_group(uint64_t t, uint64_t n,
 // enqueue of that form (no scratch, no order: every track has its own warp).
 bool use_group(const dprop_launch* lc, const dprop_detector* det,
                const dprop_config& cfg, uint64_t n);
-// Runs every fp32 kernel of that form on no track: the driver loads its code
-// and reserves its local memory now, not at the first call that takes it.
-dprop_status load_group_forms(cudaStream_t stream);
+// Has the driver load the code of every fp32 kernel of that form now, not at
+// the first call that takes it.
+dprop_status load_group_forms();
 // Whether the launch leaves its shape open (method and sort apart).
 bool open_shape(const dprop_launch* lc);
 template <typename In>
